@@ -189,46 +189,11 @@ __device__ __forceinline__ float edge_eval(float nx, float ny, float px, float p
     return s;
 }
 
-// edge_eval without the leading 0.0 + : the same value except that an exact zero can come out
-// as -0.0 instead of +0.0, which no edge test (e > 0, e < 0, tie rule) can tell apart, nor the
-// sample depth computed from it (interp_depth_fast). The coverage loop's form.
-__device__ __forceinline__ float edge_eval_test(float nx, float ny, float px, float py, float x, float y) {
-    const float dx = x - px, dy = y - py;
-    return nx * dx + ny * dy;
-}
-
 // EdgeFunctions::inside for one edge (src/rasterizer/mod.rs:148-170) without branches: pass
 // when the value is positive, or when it is zero (or NaN) and the tie rule holds; the tie rule
 // keys off the normal: x > 0, or x not negative and y < 0 (edge_tie, once per triangle edge).
 __device__ __forceinline__ bool edge_tie(float nx, float ny) { return (nx > 0.0f) | (!(nx < 0.0f) & (ny < 0.0f)); }
 __device__ __forceinline__ bool edge_pass_t(float e, bool tie) { return (e > 0.0f) | (!(e < 0.0f) & tie); }
-
-// clamp01 that returns a NaN as a NaN of unspecified payload and may return +0.0 for -0.0
-// (max.NaN / min.NaN: two instructions).
-__device__ __forceinline__ float clamp01_nan(float x) {
-    float r;
-    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
-    asm("min.NaN.f32 %0, %1, 0f3F800000;" : "=f"(r) : "f"(r));
-    return r;
-}
-
-// RasterizerTriangle::fragment's interpolate_depth (src/rasterizer/mod.rs:226-236):
-// b0 = clamp(e1 inv), b1 = clamp(e2 inv), b2 = clamp((1 - b0) - b1), z = (b0 z0 + b1 z1) +
-// b2 z2 with inv = 1 / triangle_2x_area, here over edge values that may carry either sign of
-// zero (edge_eval_test) and with clamp01_nan. The depth comes out bit for bit as the
-// reference's (edge values with the
-// leading 0 +, clamp01), except for the payload of a NaN (a NaN depth never passes the depth
-// test, and a shader that reads it saturates it to 0): flipping the sign of a zero b0 or b1
-// flips only the sign of a zero product b * z, and the sum can then only change from +0 to
-// -0 when another product is -0 too, which needs a corner depth of -0 -- the viewport's final
-// + zmin makes every screen depth +0 rather than -0; b2 = clamp01((1 - b0) - b1) is never -0.
-__device__ __forceinline__ float interp_depth_fast(float e1, float e2, float inv, float z0, float z1,
-                                                   float z2) {
-    const float b0 = clamp01_nan(e1 * inv);
-    const float b1 = clamp01_nan(e2 * inv);
-    const float b2 = clamp01_nan(1.0f - b0 - b1);
-    return b0 * z0 + b1 * z1 + b2 * z2;
-}
 
 // RGSS_SAMPLE_PATTERN (src/rasterizer/mod.rs:109-114); 1 sample = pixel centre (extension).
 template <int S>
@@ -240,6 +205,125 @@ template <int S>
 __device__ __forceinline__ float sample_dy(int i) {
     if (S == 1) return 0.5f;
     return i == 0 ? 1.0f / 8.0f : i == 1 ? 5.0f / 8.0f : i == 2 ? 7.0f / 8.0f : 3.0f / 8.0f;
+}
+
+// ------------------------------------------------------------------ coverage and sample depths
+
+// Two binary32 values in one 64-bit register pair: the packed add and multiply round each half
+// like the scalar instruction and take one issue slot for both.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// 1 / triangle_2x_area as cover_pixel takes it: NaN marks an item whose edge values or clamped
+// barycentrics could be NaN (a coordinate of 2^30 or more, or an infinite or NaN reciprocal);
+// its pixels take cover_exact. Below 2^30 every difference, product and sum of the edge
+// functions stays finite.
+__device__ __forceinline__ float cover_inv(const float4 s[3]) {
+    const float inv = 1.0f / tri2x_area(s[0].x, s[0].y, s[1].x, s[1].y, s[2].x, s[2].y);
+    float m = 0.0f;  // a NaN coordinate makes the reciprocal NaN
+#pragma unroll
+    for (int k = 0; k < 3; ++k) m = fmaxf(m, fmaxf(fabsf(s[k].x), fabsf(s[k].y)));
+    return (m < 0x1p30f && fabsf(inv) <= FLT_MAX) ? inv : __int_as_float(0x7FC00000);
+}
+
+template <int S>
+struct Cover {
+    uint32_t mask;  // bit k: sample k covered
+    float z[S];     // sample depths; meaningless where the sample is not covered
+};
+
+// Coverage (EdgeFunctions::eval, src/rasterizer/mod.rs:134-146) and sample depths
+// (RasterizerTriangle::fragment, mod.rs:225-253) of one pixel in the reference's own steps: any
+// input, including NaN and infinite ones. Kept out of line: cover_pixel calls it only for
+// samples exactly on an edge and for items cover_inv marks.
+template <int S>
+__device__ __noinline__ Cover<S> cover_exact(float p0x, float p0y, float p1x, float p1y, float p2x, float p2y,
+                                             float z0, float z1, float z2, float fx, float fy) {
+    Cover<S> c;
+    c.mask = 0;
+    const float inv = 1.0f / tri2x_area(p0x, p0y, p1x, p1y, p2x, p2y);
+    // inward normals (RasterizerTriangle::new, src/rasterizer/mod.rs:199-204)
+    const float n0x = -(p1y - p0y), n0y = p1x - p0x;
+    const float n1x = -(p2y - p1y), n1y = p2x - p1x;
+    const float n2x = -(p0y - p2y), n2y = p0x - p2x;
+    const bool t0 = edge_tie(n0x, n0y), t1 = edge_tie(n1x, n1y), t2 = edge_tie(n2x, n2y);
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+        const float xs = fx + sample_dx<S>(k), ys = fy + sample_dy<S>(k);
+        const float e0 = edge_eval(n0x, n0y, p0x, p0y, xs, ys);
+        const float e1 = edge_eval(n1x, n1y, p1x, p1y, xs, ys);
+        const float e2 = edge_eval(n2x, n2y, p2x, p2y, xs, ys);
+        const bool in = edge_pass_t(e0, t0) & edge_pass_t(e1, t1) & edge_pass_t(e2, t2);
+        const float b0 = clamp01(e1 * inv);
+        const float b1 = clamp01(e2 * inv);
+        const float b2 = clamp01(1.0f - b0 - b1);
+        c.mask |= (uint32_t)in << k;
+        c.z[k] = b0 * z0 + b1 * z1 + b2 * z2;
+    }
+    return c;
+}
+
+// The same coverage mask and depths, bit for bit where a sample is covered, in about half the
+// issue slots. `inv` is cover_inv's.
+//   - An edge's value (-vy) dx + vx dy, v = next point - point and d = sample - point, is
+//     vx dy - vy dx: one packed add for both differences, one packed multiply, one subtraction.
+//     Dropping the reference's leading 0 + can only turn +0 into -0.
+//   - With no NaN among the three values, the smallest decides: above 0 every edge passes, below
+//     0 one fails whatever the tie rule. Exactly 0 leaves it to the tie rule: cover_exact.
+//   - Saturating multiplies and adds are clamp01 for values that are not NaN, except that a -0
+//     comes out +0. A zero b0 or b1 of the other sign flips only the sign of a zero product
+//     b z, and the sum can only change from +0 to -0 when another product is -0 too, which needs
+//     a corner depth of -0; the viewport's final + zmin makes every screen depth +0 instead, and
+//     clamp((1 - b0) - b1) is never -0.
+// The raster kernels are bound by instruction issue (70-77% of slots). Against two compares per
+// edge, two clamps per weight and scalar edge values: the 100k-triangle soup at 1080p 341 -> 330 us
+// a frame, the 2M-triangle 4K terrain 472 -> 454 us. Packing over pairs of samples instead, or the depth
+// sums as well, gave no more (the latter is contracted to a fused multiply-add and is wrong).
+template <int S>
+__device__ __forceinline__ Cover<S> cover_pixel(float p0x, float p0y, float p1x, float p1y, float p2x, float p2y,
+                                                float inv, float z0, float z1, float z2, float fx, float fy) {
+    Cover<S> c;
+    c.mask = 0;
+    const f32x2 o = pack2(fy, fx);
+    const f32x2 m0 = pack2(-p0y, -p0x), m1 = pack2(-p1y, -p1x), m2 = pack2(-p2y, -p2x);
+    const f32x2 v0 = pack2(p1x - p0x, p1y - p0y), v1 = pack2(p2x - p1x, p2y - p1y), v2 = pack2(p0x - p2x, p0y - p2y);
+    bool exact = !(fabsf(inv) <= FLT_MAX);
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+        const f32x2 sp = add2(o, pack2(sample_dy<S>(k), sample_dx<S>(k)));  // exact
+        float a, b, e0, e1, e2;
+        unpack2(mul2(v0, add2(sp, m0)), a, b);
+        e0 = a - b;
+        unpack2(mul2(v1, add2(sp, m1)), a, b);
+        e1 = a - b;
+        unpack2(mul2(v2, add2(sp, m2)), a, b);
+        e2 = a - b;
+        const float e = fminf(fminf(e0, e1), e2);
+        c.mask |= (e > 0.0f) ? 1u << k : 0u;
+        exact |= e == 0.0f;
+        const float b0 = __saturatef(e1 * inv), b1 = __saturatef(e2 * inv);
+        const float b2 = __saturatef(1.0f - b0 - b1);
+        c.z[k] = b0 * z0 + b1 * z1 + b2 * z2;
+    }
+    if (exact) c = cover_exact<S>(p0x, p0y, p1x, p1y, p2x, p2y, z0, z1, z2, fx, fy);
+    return c;
 }
 
 // Fragment::interpolate's sample-point choice (src/rasterizer/mod.rs:70-83): pixel centre

@@ -956,7 +956,7 @@ __device__ __forceinline__ void stage_entry(RasterSmem<S, TS>& sm, const FrameDe
             sm.iuv[2 * q + 1][it] = uv[q][1];
         }
         // 1 / triangle_2x_area (RasterizerTriangle::new, src/rasterizer/mod.rs:206)
-        sm.iinv[it] = 1.0f / tri2x_area(sv[0].x, sv[0].y, sv[1].x, sv[1].y, sv[2].x, sv[2].y);
+        sm.iinv[it] = cover_inv(sv);
         uint32_t bx0, bx1, by0, by1;
         pixel_bbox(sv, f.width, f.height, bx0, bx1, by0, by1);
         const uint32_t cx0 = max(bx0, X0), cx1 = min(bx1, X0 + TS);
@@ -1104,7 +1104,7 @@ __device__ __forceinline__ void warp_depth(RasterSmem<S, TS>& sm, uint32_t w, ui
         sm.sitem[w][sq] = (uint8_t)it;
         sm.spix[w][sq] = (uint8_t)pix;
         sm.sdm[w][sq] = (uint8_t)dm;
-        sm.sz0[w][sq] = z[0];
+        sm.sz0[w][sq] = (cov & 1u) ? z[0] : 0.0f;
         shaded += __popc(dm);
         fsinv += 1;
     }
@@ -1446,29 +1446,12 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
                     const uint32_t lx = mode ? line : along, ly = mode ? along : line;
                     pix = ly * TS + lx;
                     const float fx = (float)(X0 + lx), fy = (float)(Y0 + ly);
-                    float n0x, n0y, n1x, n1y, n2x, n2y;
-                    item_normal(sm, it, 0, n0x, n0y);
-                    item_normal(sm, it, 1, n1x, n1y);
-                    item_normal(sm, it, 2, n2x, n2y);
-                    const float p0x = sm.ipx[0][it], p0y = sm.ipy[0][it];
-                    const float p1x = sm.ipx[1][it], p1y = sm.ipy[1][it];
-                    const float p2x = sm.ipx[2][it], p2y = sm.ipy[2][it];
-                    // tie rule per edge (EdgeFunctions::inside, mod.rs:148-170), once per pixel
-                    const bool t0 = edge_tie(n0x, n0y), t1 = edge_tie(n1x, n1y), t2 = edge_tie(n2x, n2y);
-                    const float inv = sm.iinv[it];
-                    const float z0 = sm.iz[0][it], z1 = sm.iz[1][it], z2 = sm.iz[2][it];
+                    const Cover<S> c = cover_pixel<S>(sm.ipx[0][it], sm.ipy[0][it], sm.ipx[1][it], sm.ipy[1][it],
+                                                      sm.ipx[2][it], sm.ipy[2][it], sm.iinv[it], sm.iz[0][it],
+                                                      sm.iz[1][it], sm.iz[2][it], fx, fy);
+                    cov = c.mask;
 #pragma unroll
-                    for (int k = 0; k < S; ++k) {
-                        const float xs = fx + sample_dx<S>(k), ys = fy + sample_dy<S>(k);
-                        const float e0 = edge_eval_test(n0x, n0y, p0x, p0y, xs, ys);
-                        const float e1 = edge_eval_test(n1x, n1y, p1x, p1y, xs, ys);
-                        const float e2 = edge_eval_test(n2x, n2y, p2x, p2y, xs, ys);
-                        // branch-free: every sample's depth is computed, the covered ones kept
-                        const bool in = edge_pass_t(e0, t0) & edge_pass_t(e1, t1) & edge_pass_t(e2, t2);
-                        const float zk = interp_depth_fast(e1, e2, inv, z0, z1, z2);
-                        cov |= (uint32_t)in << k;
-                        z[k] = in ? zk : 0.0f;
-                    }
+                    for (int q = 0; q < S; ++q) z[q] = c.z[q];
                 }
                 const uint32_t bal = __ballot_sync(0xFFFFFFFFu, cov != 0);
                 if (cov) {
@@ -1940,19 +1923,11 @@ __global__ void k_kat(int op, const unsigned char* __restrict__ in, unsigned cha
             TriSetup t;
             tri_setup(t, sv);
             // the raster kernel's coverage and sample-depth arithmetic
-            uint32_t cov = 0;
-            float d[4] = {0, 0, 0, 0};
-            for (int q = 0; q < 4; ++q) {
-                const float xs = (float)x + sample_dx<4>(q), ys = (float)y + sample_dy<4>(q);
-                float e[3];
-                for (int k = 0; k < 3; ++k) e[k] = edge_eval_test(t.nx[k], t.ny[k], t.px[k], t.py[k], xs, ys);
-                bool in3 = true;
-                for (int k = 0; k < 3; ++k) in3 = in3 && edge_pass_t(e[k], edge_tie(t.nx[k], t.ny[k]));
-                if (in3) {
-                    cov |= 1u << q;
-                    d[q] = interp_depth_fast(e[1], e[2], t.inv_area, t.z[0], t.z[1], t.z[2]);
-                }
-            }
+            const Cover<4> c = cover_pixel<4>(t.px[0], t.py[0], t.px[1], t.py[1], t.px[2], t.py[2], cover_inv(sv),
+                                              t.z[0], t.z[1], t.z[2], (float)x, (float)y);
+            const uint32_t cov = c.mask;
+            float d[4];
+            for (int q = 0; q < 4; ++q) d[q] = ((cov >> q) & 1u) ? c.z[q] : 0.0f;
             if (op == 2) {
                 uo[0] = cov;
                 for (int q = 0; q < 4; ++q) fo[1 + q] = d[q];

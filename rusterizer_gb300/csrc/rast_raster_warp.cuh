@@ -107,7 +107,7 @@ __device__ __forceinline__ void wstage_item(WItem& it, const FrameDev& f, const 
         it.uv[2 * q + 1] = uv[q][1];
     }
     // 1 / triangle_2x_area (RasterizerTriangle::new, src/rasterizer/mod.rs:206)
-    it.inv = 1.0f / tri2x_area(sv[0].x, sv[0].y, sv[1].x, sv[1].y, sv[2].x, sv[2].y);
+    it.inv = cover_inv(sv);
     uint32_t bx0, bx1, by0, by1;
     pixel_bbox(sv, f.width, f.height, bx0, bx1, by0, by1);
     const uint32_t cx0 = max(bx0, X0), cx1 = min(bx1, X0 + TS);
@@ -174,7 +174,7 @@ __device__ __forceinline__ void wdepth(WarpUnitSmem<S, TS>& sm, const WItem& my,
         sm.sitem[sq] = (uint8_t)it;
         sm.spix[sq] = (uint8_t)pix;
         sm.sdm[sq] = (uint8_t)dm;
-        sm.sz0[sq] = z[0];
+        sm.sz0[sq] = (cov & 1u) ? z[0] : 0.0f;
         shaded += __popc(dm);
         fsinv += 1;
     }
@@ -481,23 +481,10 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const float* 
                 const uint32_t ly = y0 + row;
                 pix = ly * TS + col;
                 const float fx = (float)(X0 + col), fy = (float)(Y0 + ly);
-                // inward normals (RasterizerTriangle::new, src/rasterizer/mod.rs:199-204)
-                const float n0x = -(p1y - p0y), n0y = p1x - p0x;
-                const float n1x = -(p2y - p1y), n1y = p2x - p1x;
-                const float n2x = -(p0y - p2y), n2y = p0x - p2x;
-                // tie rule per edge (EdgeFunctions::inside, mod.rs:148-170)
-                const bool t0 = edge_tie(n0x, n0y), t1 = edge_tie(n1x, n1y), t2 = edge_tie(n2x, n2y);
+                const Cover<S> cv = cover_pixel<S>(p0x, p0y, p1x, p1y, p2x, p2y, inv, z0, z1, z2, fx, fy);
+                cov = cv.mask;
 #pragma unroll
-                for (int k = 0; k < S; ++k) {
-                    const float xs = fx + sample_dx<S>(k), ys = fy + sample_dy<S>(k);
-                    const float e0 = edge_eval_test(n0x, n0y, p0x, p0y, xs, ys);
-                    const float e1 = edge_eval_test(n1x, n1y, p1x, p1y, xs, ys);
-                    const float e2 = edge_eval_test(n2x, n2y, p2x, p2y, xs, ys);
-                    const bool in = edge_pass_t(e0, t0) & edge_pass_t(e1, t1) & edge_pass_t(e2, t2);
-                    const float zk = interp_depth_fast(e1, e2, inv, z0, z1, z2);
-                    cov |= (uint32_t)in << k;
-                    z[k] = in ? zk : 0.0f;
-                }
+                for (int k = 0; k < S; ++k) z[k] = cv.z[k];
             }
             const uint32_t bal = __ballot_sync(0xFFFFFFFFu, cov != 0);
             if (cov) {
