@@ -113,9 +113,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
                 D.uv = m->uv;
                 D.rgba = m->rgba;
                 D.idx = m->idx;
-                D.tex = DJ.tex ? DJ.tex->data : nullptr;
-                D.tex_w = DJ.tex ? (uint32_t)DJ.tex->w : 0u;
-                D.tex_h = DJ.tex ? (uint32_t)DJ.tex->h : 0u;
+                if (DJ.tex) D.set_texture(DJ.tex->data, (uint32_t)DJ.tex->w, (uint32_t)DJ.tex->h);
                 D.nverts = m->nverts;
                 D.ntris = m->ntris;
                 D.vbase = (uint32_t)vtot;

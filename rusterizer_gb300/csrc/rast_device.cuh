@@ -29,6 +29,15 @@ __device__ __forceinline__ float clamp01(float x) {
     return x;
 }
 
+// clamp01 that returns a NaN as a NaN of unspecified payload and may return +0.0 for -0.0
+// (max.NaN / min.NaN: two instructions).
+__device__ __forceinline__ float clamp01_nan(float x) {
+    float r;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(r) : "f"(x));
+    asm("min.NaN.f32 %0, %1, 0f3F800000;" : "=f"(r) : "f"(r));
+    return r;
+}
+
 // ------------------------------------------------------------------ vertex stage
 
 // Vector::dot (src/math/vector.rs:17-23): sum from 0.0, in order.
@@ -231,6 +240,12 @@ __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
     return r;
 }
 
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
 // 1 / triangle_2x_area as cover_pixel takes it: NaN marks an item whose edge values or clamped
 // barycentrics could be NaN (a coordinate of 2^30 or more, or an infinite or NaN reciprocal);
 // its pixels take cover_exact. Below 2^30 every difference, product and sum of the edge
@@ -327,33 +342,42 @@ __device__ __forceinline__ Cover<S> cover_pixel(float p0x, float p0y, float p1x,
 }
 
 // Fragment::interpolate's sample-point choice (src/rasterizer/mod.rs:70-83): pixel centre
-// when every sample passed the depth test, else the first passed sample.
+// when every sample passed the depth test, else the first passed sample. The offsets, in eighths
+// of a pixel, come from a nibble per depth mask; a float of 2^20 + n has steps of 1/8, so the
+// position is exact for pixels below 2^20.
 template <int S>
 __device__ __forceinline__ void interp_point(uint32_t x, uint32_t y, uint32_t dm, float& xs,
                                              float& ys) {
-    // offsets of the first passed sample, selected without branches
-    const int i = __ffs(dm) - 1;
-    float dx = 0.5f, dy = 0.5f;
-#pragma unroll
-    for (int k = 0; k < S; ++k) {
-        dx = i == k ? sample_dx<S>(k) : dx;
-        dy = i == k ? sample_dy<S>(k) : dy;
-    }
-    const bool all = dm == (1u << S) - 1u;
-    xs = (float)x + (all ? 0.5f : dx);
-    ys = (float)y + (all ? 0.5f : dy);
+    // nibble dm: 8 x the offset of sample ffs(dm) - 1 (5, 7, 3, 1 across and 1, 5, 7, 3 down),
+    // 4 for dm = 15; one sample: always the centre
+    const uint32_t dx = S == 1 ? 4u : (uint32_t)(0x4753575157535750ull >> (4 * dm)) & 0xFu;
+    const uint32_t dy = S == 1 ? 4u : (uint32_t)(0x4517151315171510ull >> (4 * dm)) & 0xFu;
+    xs = __uint_as_float(0x49800000u + 8u * x + dx) - 1048576.0f;
+    ys = __uint_as_float(0x49800000u + 8u * y + dy) - 1048576.0f;
 }
 
-// Perspective-correct barycentrics of Fragment::interpolate (src/rasterizer/mod.rs:85-94).
-__device__ __forceinline__ void persp_bary(float e0, float e1, float e2, float w0, float w1,
-                                           float w2, float& u, float& v, float& w) {
-    float fu = e1 / w0;
-    float fv = e2 / w1;
-    float fw = e0 / w2;
-    float sum = fu + fv + fw;
-    u = clamp01(fu / sum);
-    v = clamp01(fv / sum);
-    w = clamp01(1.0f - u - v);
+// Perspective-correct barycentrics of Fragment::interpolate (src/rasterizer/mod.rs:85-94) at
+// (xs, ys). The edge values are cover_pixel's form, and clamp01_nan may turn a -0 weight into
+// +0: the sign of a zero edge value or weight reaches no colour (a sum of zeros divides to NaN
+// either way, and a zero product only changes the sign of a zero texture coordinate or channel).
+__device__ __forceinline__ void persp_bary(float p0x, float p0y, float p1x, float p1y, float p2x, float p2y,
+                                           float w0, float w1, float w2, float xs, float ys, float& u, float& v,
+                                           float& w) {
+    const f32x2 sp = pack2(ys, xs);
+    float a, b;
+    unpack2(mul2(pack2(p1x - p0x, p1y - p0y), add2(sp, pack2(-p0y, -p0x))), a, b);
+    const float e0 = a - b;
+    unpack2(mul2(pack2(p2x - p1x, p2y - p1y), add2(sp, pack2(-p1y, -p1x))), a, b);
+    const float e1 = a - b;
+    unpack2(mul2(pack2(p0x - p2x, p0y - p2y), add2(sp, pack2(-p2y, -p2x))), a, b);
+    const float e2 = a - b;
+    const float fu = e1 / w0;
+    const float fv = e2 / w1;
+    const float fw = e0 / w2;
+    const float sum = fu + fv + fw;
+    u = clamp01_nan(fu / sum);
+    v = clamp01_nan(fv / sum);
+    w = clamp01_nan(1.0f - u - v);
 }
 
 // ------------------------------------------------------------------ texture / colour
@@ -372,50 +396,87 @@ __device__ __forceinline__ uint32_t read_texel(const uint32_t* __restrict__ tex,
     return __ldg(tex + (start >> 2));
 }
 
-// Texture::sample (src/texture.rs:65-83): manual f32 bilinear filter. inv255[b] holds
-// (b as f32) / 255.0 (Color::from_rgba, src/color.rs:22-29), correctly rounded.
-__device__ __forceinline__ void tex_sample(const uint32_t* __restrict__ tex, uint32_t tw,
-                                           uint32_t th, float u, float v,
-                                           const float* inv255, float out[4], bool& oob) {
-    float x = u * (float)(uint64_t)(tw - 1);
-    float y = v * (float)(uint64_t)(th - 1);
-    uint32_t tl, tr, bl, br;
-    if (x >= 0.0f && y >= 0.0f && x <= (float)(tw - 1) && y <= (float)(th - 1) && tw < 65536u && th < 65536u) {
-        // inside the texture (every in-range uv): floor/ceil stay below the size, so there is no
-        // row wrap or read past the end, and the flat index x + y * w fits 32 bits
-        const uint32_t xf = (uint32_t)floorf(x), xc = (uint32_t)ceilf(x);
-        const uint32_t yf = (uint32_t)floorf(y), yc = (uint32_t)ceilf(y);
-        tl = __ldg(tex + xf + yf * tw);
-        tr = __ldg(tex + xc + yf * tw);
-        bl = __ldg(tex + xf + yc * tw);
-        br = __ldg(tex + xc + yc * tw);
-    } else {
-        uint64_t xf = sat_u64(floorf(x)), xc = sat_u64(ceilf(x));
-        uint64_t yf = sat_u64(floorf(y)), yc = sat_u64(ceilf(y));
-        tl = read_texel(tex, tw, th, xf, yf, oob);
-        tr = read_texel(tex, tw, th, xc, yf, oob);
-        bl = read_texel(tex, tw, th, xf, yc, oob);
-        br = read_texel(tex, tw, th, xc, yc, oob);
-    }
-    float x_f = x - truncf(x);
-    float y_f = y - truncf(y);
-    float omx = 1.0f - x_f, omy = 1.0f - y_f;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        float ctl = inv255[(tl >> (8 * k)) & 0xFFu];
-        float ctr = inv255[(tr >> (8 * k)) & 0xFFu];
-        float cbl = inv255[(bl >> (8 * k)) & 0xFFu];
-        float cbr = inv255[(br >> (8 * k)) & 0xFFu];
-        float y0 = ctl * omx + ctr * x_f;
-        float y1 = cbl * omx + cbr * x_f;
-        out[k] = y0 * omy + y1 * y_f;
-    }
-}
-
 // Color::to_argb (src/color.rs:15-20): saturating casts, OR-combined u32 shifts.
 __device__ __forceinline__ uint32_t to_argb(float r, float g, float b, float a) {
     return (sat_u32(a * 255.0f) << 24) | (sat_u32(r * 255.0f) << 16) |
            (sat_u32(g * 255.0f) << 8) | sat_u32(b * 255.0f);
+}
+
+// Texture::sample (src/texture.rs:65-83): manual f32 bilinear filter, for any texture
+// coordinate. Color::from_rgba (src/color.rs:22-29) divides each byte by 255.
+__device__ __forceinline__ void tex_sample(const uint32_t* __restrict__ tex, uint32_t tw,
+                                           uint32_t th, float u, float v, float out[4], bool& oob) {
+    const float x = u * (float)(uint64_t)(tw - 1);
+    const float y = v * (float)(uint64_t)(th - 1);
+    const uint64_t xf = sat_u64(floorf(x)), xc = sat_u64(ceilf(x));
+    const uint64_t yf = sat_u64(floorf(y)), yc = sat_u64(ceilf(y));
+    const uint32_t tl = read_texel(tex, tw, th, xf, yf, oob);
+    const uint32_t tr = read_texel(tex, tw, th, xc, yf, oob);
+    const uint32_t bl = read_texel(tex, tw, th, xf, yc, oob);
+    const uint32_t br = read_texel(tex, tw, th, xc, yc, oob);
+    const float x_f = x - truncf(x);
+    const float y_f = y - truncf(y);
+    const float omx = 1.0f - x_f, omy = 1.0f - y_f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float ctl = (float)((tl >> (8 * k)) & 0xFFu) / 255.0f;
+        const float ctr = (float)((tr >> (8 * k)) & 0xFFu) / 255.0f;
+        const float cbl = (float)((bl >> (8 * k)) & 0xFFu) / 255.0f;
+        const float cbr = (float)((br >> (8 * k)) & 0xFFu) / 255.0f;
+        const float y0 = ctl * omx + ctr * x_f;
+        const float y1 = cbl * omx + cbr * x_f;
+        out[k] = y0 * omy + y1 * y_f;
+    }
+}
+// tex_sample and to_argb for a fragment outside tex_argb's range (out of line: rare).
+__device__ __noinline__ uint32_t tex_argb_any(const uint32_t* __restrict__ tex, uint32_t tw, uint32_t th, float u,
+                                              float v, uint32_t& oobc) {
+    float c[4];
+    bool oob = false;
+    tex_sample(tex, tw, th, u, v, c, oob);
+    if (oob) ++oobc;
+    return to_argb(c[0], c[1], c[2], c[3]);
+}
+
+// One channel of two horizontally adjacent texels as binary32: a byte spliced under 2^23 by a
+// byte permute, then b / 255 correctly rounded as b hi + RN(b lo), hi + lo = 1/255 to 2^-49
+// (equal to the division for all 256 bytes; both channels per packed instruction).
+__device__ __forceinline__ f32x2 texel_pair(uint32_t t0, uint32_t t1, uint32_t sel) {
+    const f32x2 b = add2(pack2(__uint_as_float(__byte_perm(t0, 0x4B000000u, sel)),
+                               __uint_as_float(__byte_perm(t1, 0x4B000000u, sel))),
+                         pack2(-8388608.0f, -8388608.0f));
+    return fma2(b, pack2(0x1.01p-8f, 0x1.01p-8f), mul2(b, pack2(0x1.010102p-24f, 0x1.010102p-24f)));
+}
+
+// Texture::sample and Color::to_argb of one fragment: ARGB with alpha computed only when `alpha`
+// is set (the resolve ignores the samples' alpha; only a sample capture shows it), 255 otherwise.
+// xmax, ymax = size - 1. Inside the texture (every in-range uv; `small`: both sides below 65536)
+// floor and ceil stay below the size, so there is no row wrap or read past the end, and
+//   - x + 2^23 rounded down holds floor(x) in its low bits (the coordinate is not negative);
+//   - the channels lie in [0, 1 + 2^-21], so channel * 255 + 2^23 rounded down holds the byte;
+// no conversion instruction is left, and no shared table is read.
+__device__ __forceinline__ uint32_t tex_argb(const uint32_t* __restrict__ tex, uint32_t tw, uint32_t th, float xmax,
+                                             float ymax, bool small, float u, float v, bool alpha, uint32_t& oobc) {
+    const float x = u * xmax, y = v * ymax;
+    if (!(small & (x >= 0.0f) & (y >= 0.0f) & (x <= xmax) & (y <= ymax)))
+        return tex_argb_any(tex, tw, th, u, v, oobc);
+    const float tx = __fadd_rz(x, 8388608.0f), ty = __fadd_rz(y, 8388608.0f);
+    const float x_f = x - (tx - 8388608.0f), y_f = y - (ty - 8388608.0f);
+    const uint32_t at = (__float_as_uint(tx) & 0x7FFFFFu) + (__float_as_uint(ty) & 0x7FFFFFu) * tw;
+    const uint32_t right = x_f > 0.0f ? 1u : 0u, down = y_f > 0.0f ? tw : 0u;
+    const uint32_t tl = __ldg(tex + at), tr = __ldg(tex + (at + right));
+    const uint32_t bl = __ldg(tex + (at + down)), br = __ldg(tex + (at + down + right));
+    const f32x2 fx = pack2(1.0f - x_f, x_f), fy = pack2(1.0f - y_f, y_f);
+    auto channel = [&](uint32_t sel) {
+        float a, b, c, d;
+        unpack2(mul2(texel_pair(tl, tr, sel), fx), a, b);
+        unpack2(mul2(texel_pair(bl, br, sel), fx), c, d);
+        unpack2(mul2(pack2(a + b, c + d), fy), a, b);
+        return __float_as_uint(__fadd_rz((a + b) * 255.0f, 8388608.0f));
+    };
+    const uint32_t r = channel(0x7650u), g = channel(0x7651u), b = channel(0x7652u);
+    const uint32_t a = alpha ? channel(0x7653u) : 0xFFu;
+    return __byte_perm(__byte_perm(b, g, 0x0040u), __byte_perm(r, a, 0x0040u), 0x5410u);
 }
 
 // ColorBuffer::box_filter_color (src/rasterizer/buffers.rs:111-125)

@@ -167,9 +167,7 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
     D.uv = d_uv;
     D.rgba = d_rgba;
     D.idx = d_idx;
-    D.tex = d_tex;
-    D.tex_w = d_tex ? (uint32_t)tex_w : 0u;
-    D.tex_h = d_tex ? (uint32_t)tex_h : 0u;
+    if (d_tex) D.set_texture(d_tex, (uint32_t)tex_w, (uint32_t)tex_h);
     D.nverts = nverts;
     D.ntris = ntris;
     D.fs = fs_id;

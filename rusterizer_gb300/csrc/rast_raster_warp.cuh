@@ -37,7 +37,6 @@ struct alignas(16) WarpUnitSmem {
 
 template <int S, int TS>
 struct WarpRasterSmem {
-    float inv255[256];
     WarpUnitSmem<S, TS> u[kWarpUnitWarps];
 };
 
@@ -185,8 +184,7 @@ __device__ __forceinline__ void wdepth(WarpUnitSmem<S, TS>& sm, const WItem& my,
 // Fragment shader and colour write of up to 32 fragments of the shade ring, as warp_shade does
 // for k_raster; each lane reads its fragment's item from the item's lane.
 template <int S, int TS>
-__device__ __forceinline__ void wshade(WarpUnitSmem<S, TS>& sm, const WItem& my, const float* inv255,
-                                      uint32_t head, uint32_t n, const DrawDev* __restrict__ draws,
+__device__ __forceinline__ void wshade(WarpUnitSmem<S, TS>& sm, const WItem& my, uint32_t head, uint32_t n, const DrawDev* __restrict__ draws,
                                       const FrameDev& f, const Scratch& s, uint32_t X0, uint32_t Y0,
                                       uint32_t& oobc) {
     using U = WarpUnitSmem<S, TS>;
@@ -208,43 +206,34 @@ __device__ __forceinline__ void wshade(WarpUnitSmem<S, TS>& sm, const WItem& my,
     if (valid) {
         pix = sm.spix[q];
         dm = sm.sdm[q];
-        const uint32_t x = X0 + pix % TS, y = Y0 + pix / TS;
         float xs, ys;
-        interp_point<S>(x, y, dm, xs, ys);
-        float e[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            // inward normal of edge k (RasterizerTriangle::new, src/rasterizer/mod.rs:199-204)
-            const int nk = k == 2 ? 0 : k + 1;
-            const float nx = -(py[nk] - py[k]), ny = px[nk] - px[k];
-            e[k] = edge_eval(nx, ny, px[k], py[k], xs, ys);
-        }
+        interp_point<S>(X0 + pix % TS, Y0 + pix / TS, dm, xs, ys);
         float u, v, ww;
-        persp_bary(e[0], e[1], e[2], w[0], w[1], w[2], u, v, ww);
-        const DrawDev& d = draws[meta >> 8];
-        float col[4];
+        persp_bary(px[0], py[0], px[1], py[1], px[2], py[2], w[0], w[1], w[2], xs, ys, u, v, ww);
+        const ShadeDraw d = shade_draw(&draws[meta >> 8]);
         if (d.fs == 0) {
             // FS::Texture (upstream src/main.rs:214-216)
             const float tu = tuv[0] * u + tuv[2] * v + tuv[4] * ww;
             const float tv = tuv[1] * u + tuv[3] * v + tuv[5] * ww;
-            bool oob = false;
-            tex_sample(d.tex, d.tex_w, d.tex_h, tu, tv, inv255, col, oob);
-            if (oob) ++oobc;
-        } else if (d.fs == 1) {
-            // FS::Color (upstream src/main.rs:217)
-            float vc[3][4];
-            item_colours(d, f, s, tri, meta & 0xFFu, vc);
-#pragma unroll
-            for (int c = 0; c < 4; ++c) col[c] = vc[0][c] * u + vc[1][c] * v + vc[2][c] * ww;
+            argb = tex_argb(d.tex, d.tex_w, d.tex_h, d.xmax, d.ymax, d.small, tu, tv, f.dbg_color != nullptr, oobc);
         } else {
-            // FS::Debug (upstream src/main.rs:218-220): grayscale(frag_coords.depths[0])
-            const float z0 = sm.sz0[q];
-            col[0] = z0;
-            col[1] = z0;
-            col[2] = z0;
-            col[3] = 1.0f;
+            float col[4];
+            if (d.fs == 1) {
+                // FS::Color (upstream src/main.rs:217)
+                float vc[3][4];
+                item_colours(draws[meta >> 8], f, s, tri, meta & 0xFFu, vc);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) col[c] = vc[0][c] * u + vc[1][c] * v + vc[2][c] * ww;
+            } else {
+                // FS::Debug (upstream src/main.rs:218-220): grayscale(frag_coords.depths[0])
+                const float z0 = sm.sz0[q];
+                col[0] = z0;
+                col[1] = z0;
+                col[2] = z0;
+                col[3] = 1.0f;
+            }
+            argb = to_argb(col[0], col[1], col[2], col[3]);
         }
-        argb = to_argb(col[0], col[1], col[2], col[3]);
     }
     const uint32_t key = valid ? pix : 0x10000u + lane;
     const uint32_t grp = __match_any_sync(0xFFFFFFFFu, key);
@@ -316,7 +305,7 @@ __device__ __forceinline__ void wresolve(const WarpUnitSmem<S, TS>& sm, const Fr
 // into the shade ring, shading; both rings are drained before the next batch replaces the items
 // they refer to. Then the resolve.
 template <int S, int TS>
-__device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const float* inv255, const FrameDev& f,
+__device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const FrameDev& f,
                                           const DrawDev* __restrict__ draws, const Scratch& s,
                                           const uint32_t* __restrict__ bins, uint32_t nent, uint32_t mybit,
                                           uint32_t X0, uint32_t Y0, uint32_t& shaded, uint32_t& fsinv,
@@ -416,12 +405,13 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const float* 
             j = min(j, 31u);
             const float px[3] = {shfl_f(my.px[0], j), shfl_f(my.px[1], j), shfl_f(my.px[2], j)};
             const float py[3] = {shfl_f(my.py[0], j), shfl_f(my.py[1], j), shfl_f(my.py[2], j)};
+            const bool finite = fabsf(shfl_f(my.inv, j)) <= FLT_MAX;
             const uint32_t gj = __shfl_sync(0xFFFFFFFFu, geo, j);
             const uint32_t row = t - __shfl_sync(0xFFFFFFFFu, rincl - nrows, j);
             if (t < rtot) {
                 const uint32_t x0 = gj & 31u, y0 = (gj >> 5) & 31u;
                 uint32_t a0 = x0, a1 = x0 + ((gj >> 10) & 31u);
-                line_span_pts<S, TS>(px, py, 0u, y0 + row, X0, Y0, a0, a1);
+                if (finite) line_span_pts<S, TS>(px, py, 0u, y0 + row, X0, Y0, a0, a1);
                 sm.rsta[j][row] = (uint8_t)a0;
                 sm.rpre[j][row] = (uint8_t)(a1 - a0);
             }
@@ -501,7 +491,7 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const float* 
                 wdepth<S, TS>(sm, my, head, 32, stail, s, X0, Y0, shaded, fsinv);
                 head += 32;
                 if (stail - shead >= 32) {
-                    wshade<S, TS>(sm, my, inv255, shead, 32, draws, f, s, X0, Y0, oobc);
+                    wshade<S, TS>(sm, my, shead, 32, draws, f, s, X0, Y0, oobc);
                     shead += 32;
                 }
             }
@@ -509,7 +499,7 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const float* 
         if (tail != head) wdepth<S, TS>(sm, my, head, tail - head, stail, s, X0, Y0, shaded, fsinv);
         while (stail != shead) {
             const uint32_t nsh = min(stail - shead, 32u);
-            wshade<S, TS>(sm, my, inv255, shead, nsh, draws, f, s, X0, Y0, oobc);
+            wshade<S, TS>(sm, my, shead, nsh, draws, f, s, X0, Y0, oobc);
             shead += nsh;
         }
         __syncwarp();
@@ -534,8 +524,6 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 :
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     WarpRasterSmem<S, TS>& sh = *reinterpret_cast<WarpRasterSmem<S, TS>*>(smem_raw);
-    for (uint32_t i = threadIdx.x; i < 256u; i += blockDim.x) sh.inv255[i] = (float)i / 255.0f;
-    __syncthreads();
     const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
     WarpUnitSmem<S, TS>& sm = sh.u[warp];
     const uint32_t nbusy = *(volatile unsigned int*)&queue[2];
@@ -562,7 +550,7 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 :
             nent = s.tile_count[gt];
             bins = s.bins + f.bin_base + s.tile_start[gt];
         }
-        warp_unit<S, TS>(sm, sh.inv255, f, draws, s, bins, nent, 1u << sub, X0, Y0, shaded, fsinv, oobc);
+        warp_unit<S, TS>(sm, f, draws, s, bins, nent, 1u << sub, X0, Y0, shaded, fsinv, oobc);
     }
     // bins without entries: runs of kEmptyRun bins per counter update, the clear colour
     for (;;) {

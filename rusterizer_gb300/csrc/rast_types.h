@@ -79,19 +79,31 @@ enum StatSlots : int {
     STAT_COUNT = 4,
 };
 
-struct DrawDev {
+struct alignas(16) DrawDev {
     const float* pos;      // nverts * 3
     const float* uv;       // nverts * 2
     const float* rgba;     // nverts * 4 or null
     const uint32_t* idx;   // ntris * 3
+    // what the fragment shader reads, 32 bytes (two 16-byte loads)
     const uint32_t* tex;   // texture 0 (RGBA8 packed in u32), may be null unless fs == 0
     uint32_t tex_w, tex_h;
+    float tex_xmax, tex_ymax;  // tex_w - 1, tex_h - 1
+    int32_t fs;
+    uint32_t tex_small;    // both sides below 65536: texel indices fit 32 bits (tex_argb)
     uint32_t nverts, ntris;
     uint32_t vbase;        // first vertex record of this draw
     uint32_t tbase;        // first triangle index of this draw within its frame
     uint32_t frame;
-    int32_t fs;
     float mvp[16];         // (P * V) * W, row-major
+
+    void set_texture(const uint32_t* data, uint32_t w, uint32_t h) {
+        tex = data;
+        tex_w = w;
+        tex_h = h;
+        tex_xmax = (float)(uint64_t)(w - 1u);
+        tex_ymax = (float)(uint64_t)(h - 1u);
+        tex_small = w < 65536u && h < 65536u;
+    }
 };
 
 struct FrameDev {
