@@ -155,15 +155,30 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         }
         if (vtot >= 0xFFFFFFFFull || ttot >= 0xFFFFFFFFull || bin_tot >= 0xFFFFFFFFull)
             return RAST_INVALID_ARG;
+        // raster groups: consecutive frames of one (msaa, tile)
+        for (size_t i = 0, group = 0; i < frames.size(); ++group) {
+            if (group >= (size_t)kMaxRasterGroups) return RAST_CUDA_ERROR;
+            size_t j = i;
+            uint32_t tiles = 0;
+            for (; j < frames.size() && frames[j].msaa == frames[i].msaa && frames[j].ts == frames[i].ts; ++j)
+                tiles += frames[j].ntiles;
+            for (size_t k = i; k < j; ++k) {
+                frames[k].queue = (uint32_t)group;
+                frames[k].order_begin = frames[i].tile_begin;
+                frames[k].order_n = tiles;
+                frames[k].heavy_bits = E.heavy_bits[frames[i].msaa == 4 ? 1 : 0];
+            }
+            i = j;
+        }
         // scratch
         bool ok = E.vclip.reserve(vtot) && E.vscr.reserve(vtot) && E.vcode.reserve(vtot) &&
                   E.tri_rect.reserve(ttot) && E.tri_aux.reserve(ttot) &&
                   E.counts.reserve(count_tot) && E.tile_start.reserve(tile_tot) &&
-                  E.tile_count.reserve(tile_tot) && E.tile_order.reserve(tile_tot) &&
+                  E.tile_count.reserve(tile_tot) && E.tile_order.reserve((uint64_t)kOrderArrays * tile_tot) &&
                   E.bins.reserve(bin_tot) && E.qbins.reserve(qbin_tot) && E.clip_list.reserve(3ull * ttot) &&
                   E.qcount.reserve(qbin_tot ? 4ull * tile_tot : 0ull) &&
                   E.clip_store.reserve(std::max<uint64_t>(clip_est, E.clip_hint)) &&
-                  E.frame_need.reserve(frames.size());
+                  E.reserve_state(frames.size());
         if (!ok) return RAST_OOM;
         // descriptors: one pinned staging buffer, one async copy
         const size_t off_frames = 0;
@@ -196,7 +211,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
             E.desc_bytes = total;
             E.d_desc_ptr = E.d_desc.p;
         }
-        if (cudaMemsetAsync(E.d_state, 0, sizeof(DeviceState), st) != cudaSuccess) return RAST_CUDA_ERROR;
+        if (cudaMemsetAsync(E.d_state, 0, Engine::state_bytes(frames.size()), st) != cudaSuccess) return RAST_CUDA_ERROR;
 
         LaunchArgs a{};
         a.stream = st;
@@ -209,10 +224,6 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         a.vertex_blocks = (uint32_t)vblocks.size();
         a.scan_groups = group_tot;
         a.max_tiles = max_tiles;
-        if (frames.size() == 1) {
-            a.scan_order_queue = &E.d_state->queue[0];
-            a.scan_heavy_bits = E.heavy_bits[frames[0].msaa == 4 ? 1 : 0];
-        }
         Scratch& S = a.scratch;
         S.vclip = E.vclip.p;
         S.vscr = E.vscr.p;
@@ -234,7 +245,8 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         S.clip_n = &E.d_state->clip_n;
         S.status = &E.d_state->status;
         S.stats = E.d_state->stats;
-        S.frame_need = E.frame_need.p;
+        S.frame_need = E.d_need();
+        S.queues = E.d_state->queue;
         S.log = E.log_on ? E.log.p : nullptr;
         S.log_n = &E.d_state->log_n;
         S.log_cap = E.log_on ? E.log.cap / 4 : 0;
@@ -251,36 +263,40 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         if (E.profiling) cudaEventRecord(E.ev[4], st);
         // raster: one launch per (msaa, tile) group of consecutive frames; with several groups
         // (batches of mixed MSAA) they alternate between the context stream and its side stream,
-        // so one group's tail overlaps the next group's start
-        const bool multi = !frames.empty() &&
-                           (frames.front().msaa != frames.back().msaa || frames.front().ts != frames.back().ts);
+        // so one group's tail overlaps the next group's start. The group with the most triangles
+        // comes first (the persistent raster CTAs of the first launches fill the GPU; the small
+        // groups then fill the large ones' tails), and the quadrant splits come before any raster
+        // (a split has no room beside a full raster launch).
+        struct Group {
+            size_t begin, end;
+            uint64_t tris;
+        };
+        Group groups[kMaxRasterGroups];
+        int ngroups = 0;
+        for (size_t i = 0; i < frames.size(); ++i) {
+            if (i == 0 || frames[i].queue != frames[i - 1].queue) groups[ngroups++] = {i, i, 0};
+            groups[ngroups - 1].end = i + 1;
+            groups[ngroups - 1].tris += frames[i].ntris;
+        }
+        std::stable_sort(groups, groups + ngroups, [](const Group& x, const Group& y) { return x.tris > y.tris; });
+        const bool multi = ngroups > 1;
         if (multi && err == cudaSuccess) {
             if (cudaEventRecord(E.fork, st) != cudaSuccess || cudaStreamWaitEvent(E.side, E.fork, 0) != cudaSuccess)
                 err = cudaErrorUnknown;
         }
-        int group = 0;
-        for (size_t i = 0; i < frames.size() && err == cudaSuccess; ++group) {
-            if (group >= kMaxRasterGroups) {
-                err = cudaErrorInvalidValue;
-                break;
+        for (int pass = 0; pass < 2; ++pass)
+            for (int g = 0; g < ngroups && err == cudaSuccess; ++g) {
+                const FrameDev& F = frames[groups[g].begin];
+                a.stream = (g & 1) ? E.side : st;
+                a.raster_frames = a.frames + groups[g].begin;
+                a.raster_nframes = (int)(groups[g].end - groups[g].begin);
+                a.raster_tile_offset = F.order_begin;
+                a.raster_blocks = F.order_n;
+                a.raster_queue = &E.d_state->queue[kQueueSlots * F.queue];
+                a.raster_heavy_bits = F.heavy_bits;
+                a.raster_ctas_per_sm = E.ctas_per_sm[F.msaa == 4 ? 1 : 0];
+                err = pass == 0 ? launch_bin_split(a, F.ts) : launch_raster(a, F.msaa, F.ts);
             }
-            size_t j = i;
-            uint32_t blocks = 0;
-            while (j < frames.size() && frames[j].msaa == frames[i].msaa && frames[j].ts == frames[i].ts) {
-                blocks += frames[j].ntiles;
-                ++j;
-            }
-            a.stream = (multi && (group & 1)) ? E.side : st;
-            a.raster_frames = a.frames + i;
-            a.raster_nframes = (int)(j - i);
-            a.raster_tile_offset = frames[i].tile_begin;
-            a.raster_blocks = blocks;
-            a.raster_queue = &E.d_state->queue[kQueueSlots * group];
-            a.raster_heavy_bits = E.heavy_bits[frames[i].msaa == 4 ? 1 : 0];
-            a.raster_ctas_per_sm = E.ctas_per_sm[frames[i].msaa == 4 ? 1 : 0];
-            err = launch_raster(a, frames[i].msaa, frames[i].ts);
-            i = j;
-        }
         a.stream = st;
         if (multi && err == cudaSuccess) {
             if (cudaEventRecord(E.join, E.side) != cudaSuccess || cudaStreamWaitEvent(st, E.join, 0) != cudaSuccess)
@@ -289,13 +305,9 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         if (E.profiling) cudaEventRecord(E.ev[5], st);
         if (err != cudaSuccess) return RAST_CUDA_ERROR;
         if (E.sync_after) {
-            if (cudaMemcpyAsync(E.h_state, E.d_state, sizeof(DeviceState), cudaMemcpyDeviceToHost, st) !=
-                cudaSuccess)
+            if (cudaMemcpyAsync(E.h_state, E.d_state, Engine::state_bytes(frames.size()), cudaMemcpyDeviceToHost,
+                                st) != cudaSuccess)
                 return RAST_CUDA_ERROR;
-            if (frames.size() <= E.h_need.size() || E.h_need.reserve(frames.size())) {
-                cudaMemcpyAsync(E.h_need.p, E.frame_need.p, frames.size() * sizeof(unsigned long long),
-                                cudaMemcpyDeviceToHost, st);
-            }
             if (cudaStreamSynchronize(st) != cudaSuccess) return RAST_CUDA_ERROR;
             E.desc_pending = false;  // the stream drained: the staging buffer is free
             const uint32_t status = E.h_state->status;
@@ -303,7 +315,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
             if (status & ST_BIN_OVERFLOW) {
                 for (size_t k = 0; k < frames.size(); ++k) {
                     FrameJob& J = jobs[order[k]];
-                    const uint64_t need = E.h_need.p[k];
+                    const uint64_t need = E.h_need()[k];
                     if (need > frames[k].bin_cap) J.bin_hint = need + need / 4 + 1024;
                 }
                 retry = true;
@@ -313,7 +325,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
                 retry = true;
             }
             if (retry && attempt < 2) continue;
-            for (size_t k = 0; k < frames.size(); ++k) jobs[order[k]].need = E.h_need.p[k];
+            for (size_t k = 0; k < frames.size(); ++k) jobs[order[k]].need = E.h_need()[k];
             E.last_status = status;
             std::memcpy(E.last_stats, E.h_state->stats, sizeof(E.last_stats));
             if (status & ST_BIN_OVERFLOW) return RAST_BIN_OVERFLOW;

@@ -172,7 +172,8 @@ struct FrameJob {
     uint64_t need = 0;       // bins the frame used (filled after a synchronous run)
 };
 
-// Device state block reset at the start of every launch sequence.
+// Device state block reset at the start of every launch sequence; the frames' bin allocation
+// counters (Scratch::frame_need) follow it in the same buffer.
 struct DeviceState {
     uint32_t status;
     uint32_t pad;
@@ -191,14 +192,25 @@ struct Engine {
     DevBuf<unsigned long long> tri_rect;
     DevBuf<uint32_t> tri_aux, counts, tile_start, tile_count, tile_order, bins, qbins, qcount, clip_list;
     DevBuf<float> clip_store;
-    DevBuf<unsigned long long> frame_need;
     DevBuf<uint32_t> log;
     bool log_on = false;
     DevBuf<unsigned char> d_desc;
     HostBuf<unsigned char> h_desc;
-    HostBuf<unsigned long long> h_need;
+    DevBuf<unsigned char> d_block;   // DeviceState, then frame_need[]
+    HostBuf<unsigned char> h_block;  // its copy
     DeviceState* d_state = nullptr;
     DeviceState* h_state = nullptr;
+    static size_t state_bytes(size_t nframes) { return sizeof(DeviceState) + nframes * sizeof(unsigned long long); }
+    unsigned long long* d_need() const { return reinterpret_cast<unsigned long long*>(d_state + 1); }
+    const unsigned long long* h_need() const { return reinterpret_cast<const unsigned long long*>(h_state + 1); }
+    bool reserve_state(size_t nframes) {
+        const bool moved = h_block.cap < state_bytes(nframes);
+        if (!d_block.reserve(state_bytes(nframes)) || !h_block.reserve(state_bytes(nframes))) return false;
+        d_state = reinterpret_cast<DeviceState*>(d_block.p);
+        h_state = reinterpret_cast<DeviceState*>(h_block.p);
+        if (moved) std::memset(h_block.p, 0, h_block.cap);
+        return true;
+    }
     uint64_t clip_hint = 0;
     // raster settings per MSAA class ([0] MSAA 1, [1] MSAA 4): bins of >= 2^heavy_bits entries
     // are rastered CTA-wide, the others one warp per tile; persistent raster CTAs per SM (0: as
@@ -227,16 +239,14 @@ struct Engine {
 
     bool init() {
         if (cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) != cudaSuccess) return false;
-        if (cudaMalloc(&d_state, sizeof(DeviceState)) != cudaSuccess) return false;
-        if (cudaMallocHost(&h_state, sizeof(DeviceState)) != cudaSuccess) return false;
-        std::memset(h_state, 0, sizeof(DeviceState));
+        if (!reserve_state(64)) return false;
         for (auto& e : ev)
             if (cudaEventCreate(&e) != cudaSuccess) return false;
         if (cudaEventCreateWithFlags(&desc_done, cudaEventDisableTiming) != cudaSuccess) return false;
         if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) return false;
         if (cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) != cudaSuccess) return false;
         if (cudaEventCreateWithFlags(&join, cudaEventDisableTiming) != cudaSuccess) return false;
-        return h_need.reserve(64);
+        return true;
     }
     ~Engine() {
         if (stream) cudaStreamSynchronize(stream);
@@ -247,8 +257,6 @@ struct Engine {
         if (fork) cudaEventDestroy(fork);
         if (join) cudaEventDestroy(join);
         if (side) cudaStreamDestroy(side);
-        if (d_state) cudaFree(d_state);
-        if (h_state) cudaFreeHost(h_state);
         if (stream) cudaStreamDestroy(stream);
     }
 };

@@ -4,11 +4,9 @@
 //   k_bin_count    per chunk of triangles: classify, tile rectangle, per-chunk tile histogram
 //                  in shared memory (band by band for frames of more than 16384 bins)
 //   k_clip         one warp per triangle that straddles a clip plane: clip, fan boxes, counts
-//   k_scan_cols    per tile: exclusive prefix of the histograms over chunks
-//   k_scan_tiles   per frame: exclusive prefix over tiles -> bin ranges, capacity check; for a
-//                  one-frame run also the raster tile queue
+//   k_scan_cols    per tile: exclusive prefix of the histograms over chunks; per 32 tiles: their bin
+//                  ranges, capacity check, and their places in the raster tile queue
 //   k_bin_scatter  per chunk: order-preserving scatter of triangle ids into tile bins
-//   k_tile_order   per raster launch of a batch: the raster tile queue, heaviest first
 //   k_bin_split    per 32-pixel bin: its entries split into four 16-pixel quadrant lists
 //   k_raster<S,TS> per raster tile, a CTA of 4 warps: replays the tile's triangles in
 //                  submission order with all colour/depth samples in shared memory; coverage,
@@ -413,7 +411,65 @@ __global__ void __launch_bounds__(256, 8) k_bin_count(const ChunkDev* __restrict
 
 // ===================================================================== binning: scans
 
-// One block per 32-tile group of a frame; 32 segments of chunks per tile.
+// Class of a bin in its raster queue by the bit length of its entry count: 0 without entries, then
+// steps at 1, 4, 16, 32, 64, ... 4096 entries; the step nearest to the heavy limit 2^heavy_bits is
+// moved onto it where none lies there, so that the heavy bins are whole classes (heavy_class and up).
+// Steps of 2 where most bins lie: the queue's end is then filled with small tiles (steps of 4 made the
+// 100k-triangle soup at 1080p 3% slower).
+__device__ __forceinline__ uint32_t order_class(uint32_t count, uint32_t heavy_bits) {
+    const uint32_t b = 32 - __clz(count), h = heavy_bits + 1;
+    const uint32_t s2 = h == 2 ? 2u : 3u, s3 = h == 4 ? 4u : 5u, s11 = h >= 13 && h <= 31 ? h : 13u;
+    if (b >= 5) return b >= s11 ? 11u : min(b, 12u) - 2u;
+    return (b >= 1) + (b >= s2) + (b >= s3);
+}
+// Lowest class whose bins are rastered CTA-wide.
+__device__ __forceinline__ uint32_t heavy_class(uint32_t heavy_bits) {
+    const uint32_t h = heavy_bits + 1;
+    return h >= 32 ? (uint32_t)kClasses : h >= 13 ? 11u : h >= 5 ? h - 2u : h >= 4 ? 3u : h >= 2 ? 2u : 1u;
+}
+// Place of the k-th bin of class c in the group's arrays of n tiles: two classes share an array and
+// grow towards each other from its ends.
+__device__ __forceinline__ unsigned long long order_slot(uint32_t c, uint32_t k, uint32_t n) {
+    return (unsigned long long)(c >> 1) * n + ((c & 1u) ? k : n - 1 - k);
+}
+
+// Called by one warp whose lane holds bin t of frame f (live lanes) and its entry count: allocates
+// the bins' ranges in one step (the ranges of a frame lie in no particular order), checks the
+// capacity and lists the bins in the raster queue. A prefix over a frame's tiles and a sort
+// of them took two one-CTA kernels before (2M-triangle 4K terrain 13 us, 20 scenes 54 us).
+__device__ __forceinline__ void place_bins(const FrameDev& f, uint32_t frame, const Scratch& s, uint32_t t, bool live,
+                                           uint32_t count) {
+    const uint32_t lane = lane_id();
+    uint32_t incl = live ? count : 0u;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+    // the two allocations are independent: both in flight before either result is used
+    const uint32_t c = !live            ? (uint32_t)kClasses
+                       : f.order_coarse ? (count ? 1u : 0u)
+                                        : order_class(count, f.heavy_bits);
+    const uint32_t peers = __match_any_sync(0xFFFFFFFFu, c), leader = __ffs(peers) - 1;
+    unsigned long long base = 0;
+    uint32_t slot = 0;
+    if (lane == 0 && total) base = atomicAdd(&s.frame_need[frame], (unsigned long long)total);
+    if (live && lane == leader)
+        slot = atomicAdd(&s.queues[kQueueSlots * f.queue + kQueueClass + c], (unsigned)__popc(peers));
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    slot = __shfl_sync(0xFFFFFFFFu, slot, leader) + __popc(peers & lanemask_lt());
+    if (lane == 0 && base + total > f.bin_cap) atomicOr(s.status, ST_BIN_OVERFLOW);
+    if (live) {
+        const uint32_t gt = f.tile_begin + t;
+        s.tile_count[gt] = count;
+        s.tile_start[gt] = (uint32_t)base + incl - count;
+        s.tile_order[(unsigned long long)kOrderArrays * f.order_begin + order_slot(c, slot, f.order_n)] = gt;
+    }
+}
+
+// One block per 32-tile group of a frame; 32 segments of chunks per tile: the exclusive prefix of
+// each tile's counts over the chunks, then the tiles' bin ranges (place_bins).
 __global__ void __launch_bounds__(1024) k_scan_cols(const FrameDev* __restrict__ frames,
                                                     int nframes, Scratch s) {
     pdl_enter();
@@ -440,16 +496,16 @@ __global__ void __launch_bounds__(1024) k_scan_cols(const FrameDev* __restrict__
         for (uint32_t r = r0; r < r1; ++r) sum += base[(unsigned long long)r * nt + t];
     part[seg][tl] = sum;
     __syncthreads();
+    uint32_t count = 0;
     if (seg == 0) {
-        uint32_t run = 0;
         for (int k = 0; k < 32; ++k) {
             uint32_t c = part[k][tl];
-            part[k][tl] = run;
-            run += c;
+            part[k][tl] = count;
+            count += c;
         }
-        if (t < nt) s.tile_count[f.tile_begin + t] = run;
     }
     __syncthreads();
+    if (seg == 0) place_bins(f, (uint32_t)s_frame, s, t, t < nt, count);
     if (t < nt) {
         uint32_t run = part[seg][tl];
         for (uint32_t r = r0; r < r1; ++r) {
@@ -460,44 +516,6 @@ __global__ void __launch_bounds__(1024) k_scan_cols(const FrameDev* __restrict__
             if (c) *p = run;
             run += c;
         }
-    }
-}
-
-__device__ void tile_order_block(uint32_t tile0, uint32_t n, const uint32_t* __restrict__ tile_count,
-                                 uint32_t* __restrict__ order, unsigned int* __restrict__ queue, bool overflow,
-                                 uint32_t heavy_bits, uint32_t* cnt, uint32_t* off);
-
-// One block (1024 threads) per frame: tile_start = exclusive prefix of tile_count, capacity
-// check. For a run of one frame (order_queue set) the block also builds the raster tile queue
-// (tile_order_block), which saves the separate k_tile_order launch.
-__global__ void __launch_bounds__(1024) k_scan_tiles(const FrameDev* __restrict__ frames,
-                                                     Scratch s, uint32_t* __restrict__ order,
-                                                     unsigned int* __restrict__ order_queue,
-                                                     uint32_t heavy_bits) {
-    pdl_enter();
-    __shared__ uint32_t tmp[33];
-    __shared__ uint32_t cnt[33], off[33];
-    const FrameDev& f = frames[blockIdx.x];
-    const uint32_t nt = f.ntiles;
-    const uint32_t per = (nt + blockDim.x - 1) / blockDim.x;
-    const uint32_t a = threadIdx.x * per, b = min(nt, a + per);
-    uint32_t loc = 0;
-    for (uint32_t t = a; t < b; ++t) loc += s.tile_count[f.tile_begin + t];
-    uint32_t total;
-    uint32_t run = block_excl_scan(loc, tmp, total);
-    for (uint32_t t = a; t < b; ++t) {
-        uint32_t c = s.tile_count[f.tile_begin + t];
-        s.tile_start[f.tile_begin + t] = run;
-        run += c;
-    }
-    if (threadIdx.x == 0) {
-        s.frame_need[blockIdx.x] = total;
-        if ((unsigned long long)total > f.bin_cap) atomicOr(s.status, ST_BIN_OVERFLOW);
-    }
-    if (order_queue) {
-        __syncthreads();  // every tile_count read above is done before the queue is built
-        tile_order_block(f.tile_begin, nt, s.tile_count, order, order_queue,
-                         (unsigned long long)total > f.bin_cap, heavy_bits, cnt, off);
     }
 }
 
@@ -739,6 +757,64 @@ constexpr int kRasterCtasPerSm = 7;  // occupancy the launch bounds aim at (shar
 constexpr int kEmptyRun = 8;  // bins without entries taken per queue update
 constexpr uint32_t kTrimMin = 4;  // shortest box line that line_span trims
 
+// A raster group's queue as its consumers read it: the classes' counts turned into ends (heaviest
+// class first). After a bin overflow every tile counts as empty: each is cleared, and the host runs the
+// frame again.
+struct TileQueue {
+    const uint32_t* order;  // the group's lists
+    uint32_t n, first;      // tiles of the group, the first of them
+    uint32_t end[kClasses - 1];  // bins of class 11, of 11 and 10, ...
+    uint32_t busy, empty;
+    bool overflow;
+};
+// The first warp fills it (one counter per lane, one trip to memory), then a block barrier.
+__device__ __forceinline__ void load_queue(TileQueue& tq, const unsigned int* queue, const uint32_t* order, uint32_t n,
+                                           const uint32_t* status, uint32_t first_tile) {
+    if (threadIdx.x < 32) {
+        const uint32_t lane = threadIdx.x;
+        const uint32_t st = *(volatile const uint32_t*)status;
+        const uint32_t own = lane < (uint32_t)kClasses
+                                 ? ((volatile const unsigned int*)queue)[kQueueClass + kClasses - 1 - lane] : 0u;
+        const bool overflow = (st & ST_BIN_OVERFLOW) != 0;
+        uint32_t incl = lane < (uint32_t)(kClasses - 1) && !overflow ? own : 0u;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= (uint32_t)o) incl += y;
+        }
+        if (lane < (uint32_t)(kClasses - 1)) tq.end[lane] = incl;
+        if (lane == (uint32_t)(kClasses - 1)) {
+            tq.order = order;
+            tq.n = n;
+            tq.first = first_tile;
+            tq.busy = incl;
+            tq.empty = overflow ? n : own;
+            tq.overflow = overflow;
+        }
+    }
+    __syncthreads();
+}
+// The i-th tile with entries (i < busy), heaviest class first.
+__device__ __forceinline__ uint32_t busy_tile(const TileQueue& tq, uint32_t i) {
+    uint32_t c = kClasses - 1, start = 0;
+#pragma unroll
+    for (int k = 0; k < kClasses - 2; ++k)
+        if (i >= tq.end[k]) {
+            c = kClasses - 2 - k;
+            start = tq.end[k];
+        }
+    return tq.order[order_slot(c, i - start, tq.n)];
+}
+// The i-th tile without entries (i < empty).
+__device__ __forceinline__ uint32_t empty_tile(const TileQueue& tq, uint32_t i) {
+    return tq.overflow ? tq.first + i : tq.order[order_slot(0, i, tq.n)];
+}
+// Bins in the heavy classes: the first of the queue.
+__device__ __forceinline__ uint32_t heavy_tiles(const TileQueue& tq, uint32_t heavy_bits) {
+    const uint32_t h = heavy_class(heavy_bits);
+    return h >= (uint32_t)kClasses ? 0u : tq.end[kClasses - 1 - h];
+}
+
 // A raster CTA owns one TS x TS tile: a whole bin (bin edge == TS) or one quadrant of a bin
 // twice as wide. Bin entries carry, in their low 4 bits, the quadrants the triangle's pixel box
 // touches, so a quadrant CTA skips the other entries without loading them.
@@ -786,7 +862,8 @@ struct alignas(16) RasterSmem {
     float sz0[kRasterWarps][C::QC];
     int rowd[TS + 1], cold[TS + 1];  // candidate work of the batch, difference arrays
     uint32_t tmp[40];
-    uint32_t misc[8];  // [0] tile ticket, [1] items staged, [2..4] statistics
+    uint32_t misc[8];  // [0] unit ticket, [1] items staged, [2..4] statistics, [5] the unit's bin
+    TileQueue tq;
     uint32_t zmaxw[kRasterWarps];  // per warp: largest stored depth of its share of the tile
 };
 
@@ -1236,8 +1313,8 @@ __device__ __forceinline__ void clear_tile_warp(const FrameDev& f, uint32_t x0, 
 }
 
 // Persistent raster kernel for the heavy tiles. Units are (bin, quadrant) pairs of the first
-// queue[3] bins of the raster queue (the bins with the most entries; the others go one warp per
-// tile to k_raster_warp), taken heaviest bin first from queue[0]; per unit the CTA replays the
+// bins of the raster queue (those of the heavy classes; the others go one warp per
+// tile to k_raster_warp), taken heaviest class first from queue[0]; per unit the CTA replays the
 // bin in submission order in batches of up to IC items: stage the items (A), split the tile's rows or columns over the warps by work
 // (B), then each warp walks the candidate pixels of its items inside its range — coverage
 // (EdgeFunctions::eval, mod.rs:134-146) and sample depths (RasterizerTriangle::fragment,
@@ -1247,7 +1324,7 @@ template <int S, int TS>
 __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(const FrameDev* __restrict__ frames,
                                                            int nframes,
                                                            const uint32_t* __restrict__ order,
-                                                           uint32_t ntotal, uint32_t nsx,
+                                                           uint32_t ntotal, uint32_t first_tile, uint32_t nsx,
                                                            unsigned int* __restrict__ queue,
                                                            const DrawDev* __restrict__ draws,
                                                            Scratch s) {
@@ -1257,19 +1334,23 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
     RasterSmem<S, TS>& sm = *reinterpret_cast<RasterSmem<S, TS>*>(smem_raw);
     const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
     uint32_t shaded = 0, fsinv = 0, oobc = 0;
-    const uint32_t nbusy = *(volatile unsigned int*)&queue[2];  // written by k_tile_order
-    const uint32_t nheavy = *(volatile unsigned int*)&queue[3];  // the first nheavy bins of the queue
     const uint32_t nsub = nsx * nsx;
+    load_queue(sm.tq, queue, order, ntotal, s.status, first_tile);
 
-    // unit tickets (heaviest first); the next one is taken when the current unit starts its
+    // unit tickets (heaviest bins first); the next one is taken when the current unit starts its
     // resolve, so the queue update is in flight during the resolve
-    if (threadIdx.x == 0) sm.misc[0] = atomicAdd(&queue[0], 1u);
+    const uint32_t nunits = heavy_tiles(sm.tq, frames[0].heavy_bits) * nsub;
+    if (threadIdx.x == 0) {
+        const uint32_t qi = atomicAdd(&queue[0], 1u);
+        sm.misc[0] = qi;
+        if (qi < nunits) sm.misc[5] = busy_tile(sm.tq, qi / nsub);
+    }
     for (;;) {
     __syncthreads();
-    // misc[0] is written again only after this unit's resolve, many barriers later
+    // misc[0] and misc[5] are written again only after this unit's resolve, many barriers later
     const uint32_t qi = sm.misc[0];
-    if (qi >= nheavy * nsub) break;
-    const uint32_t gt = order[qi / nsub], sub = qi % nsub;
+    if (qi >= nunits) break;
+    const uint32_t gt = sm.misc[5], sub = qi % nsub;
     const FrameDev& f = frames[frame_of_tile(frames, nframes, gt)];
     const uint32_t lt = gt - f.tile_begin;
     const uint32_t X0 = (lt % f.tiles_x) * (uint32_t)f.ts + (sub % nsx) * TS;
@@ -1479,7 +1560,10 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
             }
         }
     }
-    if (threadIdx.x == 0) sm.misc[0] = next_ticket;
+    if (threadIdx.x == 0) {
+        sm.misc[0] = next_ticket;
+        if (next_ticket < nunits) sm.misc[5] = busy_tile(sm.tq, next_ticket / nsub);
+    }
     }  // units with entries
 
     // ---- bins without entries: warps take runs of kEmptyRun bins (one counter update per run,
@@ -1487,11 +1571,11 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
     for (;;) {
         uint32_t q0 = 0;
         if (lane == 0) q0 = atomicAdd(&queue[1], (unsigned)kEmptyRun);
-        q0 = __shfl_sync(0xFFFFFFFFu, q0, 0) + nbusy;
-        if (q0 >= ntotal) break;
-        const uint32_t q1 = min(q0 + (uint32_t)kEmptyRun, ntotal);
+        q0 = __shfl_sync(0xFFFFFFFFu, q0, 0);
+        if (q0 >= sm.tq.empty) break;
+        const uint32_t q1 = min(q0 + (uint32_t)kEmptyRun, sm.tq.empty);
         for (uint32_t qi = q0; qi < q1; ++qi) {
-            const uint32_t gt = order[qi];
+            const uint32_t gt = empty_tile(sm.tq, qi);
             const FrameDev& f = frames[frame_of_tile(frames, nframes, gt)];
             const uint32_t lt = gt - f.tile_begin;
             const uint32_t edge = (uint32_t)f.ts;
@@ -1524,20 +1608,23 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
 
 // Splits each 32-pixel bin with entries into its four quadrant lists, keeping submission
 // order within each (an entry goes to every quadrant its mask names). Persistent CTAs walk the
-// bins with entries in the raster queue's order (k_tile_order runs first); the quadrant raster
+// bins with entries in the raster queue's order; the quadrant raster
 // CTAs then read only their own entries. Windows of 4 consecutive entries per thread; the
 // per-quadrant counts travel as 16-bit fields (two quadrants per word) through one block scan.
 __global__ void __launch_bounds__(256) k_bin_split(const FrameDev* __restrict__ frames, int nframes,
-                                                   const uint32_t* __restrict__ order,
+                                                   const uint32_t* __restrict__ order, uint32_t ntotal,
+                                                   uint32_t first_tile,
                                                    const unsigned int* __restrict__ queue, Scratch s) {
     pdl_enter();
     constexpr int kPer = 4;
+    __shared__ TileQueue tq;
+    load_queue(tq, queue, order, ntotal, s.status, first_tile);
     __shared__ uint32_t tmp[2][33];
     __shared__ uint32_t base[4];
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const uint32_t nbusy = *(volatile const unsigned int*)&queue[2];
+    const uint32_t nbusy = tq.busy;
     for (uint32_t qi = blockIdx.x; qi < nbusy; qi += gridDim.x) {
-        const uint32_t gt = order[qi];
+        const uint32_t gt = busy_tile(tq, qi);
         const uint32_t n = s.tile_count[gt];
         const FrameDev& f = frames[frame_of_tile(frames, nframes, gt)];
         const unsigned long long start = s.tile_start[gt];
@@ -1606,61 +1693,6 @@ __global__ void __launch_bounds__(256) k_bin_split(const FrameDev* __restrict__ 
         if (threadIdx.x < 4) s.qcount[4ull * gt + threadIdx.x] = base[threadIdx.x];
         __syncthreads();
     }
-}
-
-// Tile queue of one raster launch (block-wide, 1024 threads): tiles with entries first, in
-// decreasing order of entry count (bucketed by bit length), then tiles without entries;
-// queue[2] = tiles with entries, queue[3] = the leading tiles with at least 2^heavy_bits entries
-// (rastered CTA-wide by k_raster; the rest one warp per tile by k_raster_warp). After a bin
-// overflow every tile counts as empty (each is cleared and the host re-runs the frame).
-__device__ void tile_order_block(uint32_t tile0, uint32_t n, const uint32_t* __restrict__ tile_count,
-                                 uint32_t* __restrict__ order, unsigned int* __restrict__ queue, bool overflow,
-                                 uint32_t heavy_bits, uint32_t* cnt, uint32_t* off) {
-    if (threadIdx.x < 33) cnt[threadIdx.x] = 0;
-    __syncthreads();
-    // lanes with the same bucket add once per warp (thousands of tiles share a few buckets)
-    for (uint32_t i0 = 0; i0 < n; i0 += blockDim.x) {
-        const uint32_t i = i0 + threadIdx.x;
-        const uint32_t b = i < n ? 32 - __clz(overflow ? 0u : tile_count[tile0 + i]) : 33u;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, b);
-        if (b < 33u && lane_id() == (uint32_t)(__ffs(peers) - 1)) atomicAdd(&cnt[b], (uint32_t)__popc(peers));
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = 0, heavy = 0;
-        for (int b = 32; b >= 0; --b) {
-            off[b] = run;
-            run += cnt[b];
-            // bins of at least 2^heavy_bits entries (bit length above heavy_bits), never empty ones
-            if (b > (int)heavy_bits && b > 0) heavy += cnt[b];
-        }
-        queue[2] = n - cnt[0];
-        queue[3] = heavy;
-    }
-    __syncthreads();
-    for (uint32_t i0 = 0; i0 < n; i0 += blockDim.x) {
-        const uint32_t i = i0 + threadIdx.x;
-        const uint32_t b = i < n ? 32 - __clz(overflow ? 0u : tile_count[tile0 + i]) : 33u;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, b);
-        const uint32_t leader = __ffs(peers) - 1;
-        uint32_t base = 0;
-        if (b < 33u && lane_id() == leader) base = atomicAdd(&off[b], (uint32_t)__popc(peers));
-        base = __shfl_sync(0xFFFFFFFFu, base, leader);
-        if (b < 33u) order[tile0 + base + __popc(peers & lanemask_lt())] = tile0 + i;
-    }
-}
-
-// The tile queue of one raster launch over a group of frames (tile_order_block). One block.
-__global__ void __launch_bounds__(1024) k_tile_order(uint32_t tile0, uint32_t n,
-                                                     const uint32_t* __restrict__ tile_count,
-                                                     uint32_t* __restrict__ order,
-                                                     unsigned int* __restrict__ queue,
-                                                     const uint32_t* __restrict__ status,
-                                                     uint32_t heavy_bits) {
-    pdl_enter();
-    __shared__ uint32_t cnt[33], off[33];
-    const bool overflow = (*(volatile const uint32_t*)status & ST_BIN_OVERFLOW) != 0;
-    tile_order_block(tile0, n, tile_count, order, queue, overflow, heavy_bits, cnt, off);
 }
 
 // ===================================================================== launchers
@@ -1751,35 +1783,22 @@ static cudaError_t launch_raster_t(const LaunchArgs& a, uint32_t nsx) {
         wgrid_cap = wgrid_cap < cap ? wgrid_cap : cap;
     }
     if (a.raster_blocks == 0) return cudaSuccess;
-    if (!a.scan_order_queue) {  // else k_scan_tiles built the queue
-        e = launch_pdl(k_tile_order, 1, 1024, 0, a.stream, a.raster_tile_offset, a.raster_blocks,
-                       a.scratch.tile_count, a.scratch.tile_order, a.raster_queue, a.scratch.status,
-                       a.raster_heavy_bits);
-        if (e != cudaSuccess) return e;
-    }
-    if (nsx > 1) {
-        const unsigned sgrid = a.raster_blocks < (uint32_t)grid_cap ? a.raster_blocks : (unsigned)grid_cap;
-        e = launch_pdl(k_bin_split, sgrid, 256, 0, a.stream, a.raster_frames, a.raster_nframes,
-                       (const uint32_t*)(a.scratch.tile_order + a.raster_tile_offset),
-                       (const unsigned int*)a.raster_queue, a.scratch);
-        if (e != cudaSuccess) return e;
-    }
+    const uint32_t* order = a.scratch.tile_order + (unsigned long long)kOrderArrays * a.raster_tile_offset;
     const unsigned long long units = (unsigned long long)a.raster_blocks * nsx * nsx;
     // heavy tiles CTA-wide (none when every bin is below the threshold: the launch then only
     // helps with the bins without entries), then the light tiles one warp each
     if (a.raster_heavy_bits < 32) {
         const unsigned grid = units < (unsigned long long)grid_cap ? (unsigned)units : (unsigned)grid_cap;
         e = launch_pdl(k_raster<S, TS>, grid, kRasterThreads, bytes, a.stream, a.raster_frames, a.raster_nframes,
-                       (const uint32_t*)(a.scratch.tile_order + a.raster_tile_offset), a.raster_blocks, nsx,
-                       a.raster_queue, a.draws, a.scratch);
+                       order, a.raster_blocks, a.raster_tile_offset, nsx, a.raster_queue, a.draws, a.scratch);
         if (e != cudaSuccess) return e;
     }
     if (a.raster_heavy_bits == 0) return cudaSuccess;  // every bin with entries is heavy
     const unsigned long long wunits = (units + kWarpUnitWarps - 1) / kWarpUnitWarps;
     const unsigned wgrid = wunits < (unsigned long long)wgrid_cap ? (unsigned)wunits : (unsigned)wgrid_cap;
     return launch_pdl(k_raster_warp<S, TS>, wgrid, 32 * kWarpUnitWarps, wbytes, a.stream, a.raster_frames,
-                      a.raster_nframes, (const uint32_t*)(a.scratch.tile_order + a.raster_tile_offset),
-                      a.raster_blocks, nsx, a.raster_queue, a.draws, a.scratch);
+                      a.raster_nframes, order, a.raster_blocks, a.raster_tile_offset, nsx, a.raster_queue, a.draws,
+                      a.scratch);
 }
 
 cudaError_t launch_vertex(const LaunchArgs& a) {
@@ -1817,20 +1836,23 @@ cudaError_t launch_bin_count(const LaunchArgs& a) {
 }
 
 cudaError_t launch_scans(const LaunchArgs& a) {
-    if (a.scan_groups) {
-        cudaError_t e = launch_pdl(k_scan_cols, a.scan_groups, 1024, 0, a.stream, a.frames, a.nframes, a.scratch);
-        if (e != cudaSuccess) return e;
-    }
-    if (a.nframes)
-        return launch_pdl(k_scan_tiles, (unsigned)a.nframes, 1024, 0, a.stream, a.frames, a.scratch,
-                          a.scratch.tile_order, a.scan_order_queue, a.scan_heavy_bits);
-    return cudaSuccess;
+    if (a.scan_groups == 0) return cudaSuccess;
+    return launch_pdl(k_scan_cols, a.scan_groups, 1024, 0, a.stream, a.frames, a.nframes, a.scratch);
 }
 
 cudaError_t launch_bin_scatter(const LaunchArgs& a) {
     if (a.nchunks == 0) return cudaSuccess;
     return launch_pdl(k_bin_scatter, a.nchunks, kScatterThreads, 0, a.stream, a.chunks, a.draws, a.frames,
                       a.scratch);
+}
+
+cudaError_t launch_bin_split(const LaunchArgs& a, int ts) {
+    if (raster_edge(ts) == ts || a.raster_blocks == 0) return cudaSuccess;
+    const uint32_t cap = 8u * (uint32_t)sm_count();  // resident CTAs (2048 threads per SM)
+    return launch_pdl(k_bin_split, a.raster_blocks < cap ? a.raster_blocks : cap, 256, 0, a.stream, a.raster_frames,
+                      a.raster_nframes,
+                      (const uint32_t*)(a.scratch.tile_order + (unsigned long long)kOrderArrays * a.raster_tile_offset),
+                      a.raster_blocks, a.raster_tile_offset, (const unsigned int*)a.raster_queue, a.scratch);
 }
 
 cudaError_t launch_raster(const LaunchArgs& a, int msaa, int ts) {

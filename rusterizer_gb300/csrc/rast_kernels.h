@@ -20,10 +20,6 @@ struct LaunchArgs {
     uint32_t vertex_blocks;
     uint32_t scan_groups;  // 32-tile groups over all frames
     uint32_t max_tiles;    // largest per-frame tile count
-    // a run of one frame: k_scan_tiles builds the raster tile queue into these counters (with
-    // this heavy-tile threshold) and the raster launch skips k_tile_order; null otherwise
-    unsigned int* scan_order_queue;
-    uint32_t scan_heavy_bits;
     // raster launch over one (msaa, tile) group of consecutive frames
     const FrameDev* raster_frames;
     int raster_nframes;
@@ -39,6 +35,7 @@ cudaError_t launch_vertex(const LaunchArgs& a);
 cudaError_t launch_bin_count(const LaunchArgs& a);
 cudaError_t launch_scans(const LaunchArgs& a);
 cudaError_t launch_bin_scatter(const LaunchArgs& a);
+cudaError_t launch_bin_split(const LaunchArgs& a, int ts);  // 32-pixel bins: before launch_raster
 cudaError_t launch_raster(const LaunchArgs& a, int msaa, int ts);
 size_t raster_smem(int msaa, int ts);
 unsigned long long kernel_launches();

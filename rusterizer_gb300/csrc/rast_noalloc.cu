@@ -79,15 +79,16 @@ struct Carve {
 // clip-store capacities; `end` is the bytes used.
 struct Layout {
     size_t state, frame, draw, chunks, vblocks, vclip, vscr, vcode, rect, aux, counts, tstart, tcount,
-        torder, need, bins, qbins, qcount, clip, clist, end;
+        torder, bins, qbins, qcount, clip, clist, end;
 };
 
 Layout carve_layout(uint32_t nverts, uint32_t ntris, uint32_t nchunks, uint32_t nvb, uint32_t ntiles,
-                    bool split, unsigned long long bin_cap, unsigned long long clip_floats) {
+                    bool split, unsigned long long bin_cap, unsigned long long clip_floats,
+                    bool coarse) {
     using namespace rast;
     Carve c;
     Layout L;
-    L.state = c.take(sizeof(DeviceState));
+    L.state = c.take(sizeof(DeviceState) + sizeof(unsigned long long));  // and frame_need
     L.frame = c.take(sizeof(FrameDev));
     L.draw = c.take(sizeof(DrawDev));
     L.chunks = c.take(sizeof(ChunkDev) * (nchunks ? nchunks : 1));
@@ -100,8 +101,7 @@ Layout carve_layout(uint32_t nverts, uint32_t ntris, uint32_t nchunks, uint32_t 
     L.counts = c.take(sizeof(uint32_t) * (size_t)nchunks * ntiles);
     L.tstart = c.take(sizeof(uint32_t) * ntiles);
     L.tcount = c.take(sizeof(uint32_t) * ntiles);
-    L.torder = c.take(sizeof(uint32_t) * ntiles);
-    L.need = c.take(sizeof(unsigned long long));
+    L.torder = c.take((coarse ? 1 : kOrderArrays) * sizeof(uint32_t) * (size_t)ntiles);
     L.bins = c.take(sizeof(uint32_t) * bin_cap);
     // 32-pixel bins are split into quadrant lists for the raster
     L.qbins = c.take(split ? sizeof(uint32_t) * 4ull * bin_cap : 0);
@@ -161,6 +161,8 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
     F.ntris = ntris;
     F.nchunks = nchunks;
     F.clear_depth = clear_depth;
+    F.order_n = F.ntiles;
+    F.heavy_bits = kDefaultHeavyBits;
     F.out = d_argb;
     DrawDev D{};
     D.pos = d_pos;
@@ -189,12 +191,18 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
     unsigned long long bin_cap = 4ull * ntris + F.ntiles + 1024ull;
     unsigned long long clip_floats = 32ull * ntris + 4096ull;
     for (int attempt = 0; attempt < 3; ++attempt) {
-        const Layout L = carve_layout(nverts, ntris, nchunks, nvb, F.ntiles, split, bin_cap, clip_floats);
+        // the raster queue's lists take kOrderArrays arrays, or one where the rest leaves no room for them
+        F.order_coarse = 0;
+        Layout L = carve_layout(nverts, ntris, nchunks, nvb, F.ntiles, split, bin_cap, clip_floats, false);
+        if (L.end > kNoAllocScratchBytes) {
+            F.order_coarse = 1;
+            L = carve_layout(nverts, ntris, nchunks, nvb, F.ntiles, split, bin_cap, clip_floats, true);
+        }
         if (L.end > kNoAllocScratchBytes) return RAST_INVALID_ARG;
         F.bin_cap = bin_cap;
 
         // only the state block must start at zero; every other region is written before it is read
-        bool ok = cudaMemsetAsync(base + L.state, 0, sizeof(DeviceState), st) == cudaSuccess;
+        bool ok = cudaMemsetAsync(base + L.state, 0, sizeof(DeviceState) + sizeof(unsigned long long), st) == cudaSuccess;
         ok = ok && cudaMemcpyAsync(base + L.frame, &F, sizeof(F), cudaMemcpyHostToDevice, st) == cudaSuccess;
         ok = ok && cudaMemcpyAsync(base + L.draw, &D, sizeof(D), cudaMemcpyHostToDevice, st) == cudaSuccess;
         {
@@ -236,8 +244,6 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
         a.raster_blocks = F.ntiles;
         a.raster_queue = dstate->queue;
         a.raster_heavy_bits = kDefaultHeavyBits;
-        a.scan_order_queue = dstate->queue;
-        a.scan_heavy_bits = kDefaultHeavyBits;
         Scratch& S = a.scratch;
         S.vclip = reinterpret_cast<float4*>(base + L.vclip);
         S.vscr = reinterpret_cast<float4*>(base + L.vscr);
@@ -259,7 +265,8 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
         S.clip_n = &dstate->clip_n;
         S.status = &dstate->status;
         S.stats = dstate->stats;
-        S.frame_need = reinterpret_cast<unsigned long long*>(base + L.need);
+        S.frame_need = reinterpret_cast<unsigned long long*>(dstate + 1);
+        S.queues = dstate->queue;
         S.log = nullptr;
         S.log_n = &dstate->log_n;
         S.log_cap = 0;
@@ -268,19 +275,23 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
         if (err == cudaSuccess) err = launch_bin_count(a);
         if (err == cudaSuccess) err = launch_scans(a);
         if (err == cudaSuccess) err = launch_bin_scatter(a);
+        if (err == cudaSuccess) err = launch_bin_split(a, ts);
         if (err == cudaSuccess) err = launch_raster(a, msaa, ts);
         if (err != cudaSuccess) {
             cudaGetLastError();
             return RAST_CUDA_ERROR;
         }
-        DeviceState h{};
-        unsigned long long need = 0;
-        if (cudaMemcpyAsync(&h, dstate, sizeof(h), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaMemcpyAsync(&need, base + L.need, sizeof(need), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        struct {
+            DeviceState state;
+            unsigned long long need;
+        } hs{};
+        if (cudaMemcpyAsync(&hs, dstate, sizeof(hs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess) {
             cudaGetLastError();
             return RAST_CUDA_ERROR;
         }
+        const DeviceState& h = hs.state;
+        const unsigned long long need = hs.need;
         if (h.status & (ST_BIN_OVERFLOW | ST_CLIP_STORE_OVERFLOW)) {
             if (attempt == 2) return RAST_BIN_OVERFLOW;
             if ((h.status & ST_BIN_OVERFLOW) && need > bin_cap) bin_cap = need + need / 4 + 1024;

@@ -9,9 +9,8 @@
 // arithmetic is the same device functions as k_raster (coverage, sample depths, tie rule,
 // interpolation, shaders, resolve), so results are bit-identical; only the work split differs.
 //
-// The persistent kernel takes light tiles (bins past the first `nheavy` of the raster queue,
-// which k_tile_order or, for a one-frame run, k_scan_tiles sorts heaviest first) from their own
-// counter, then helps clear the bins without entries. k_raster takes the heavy tiles.
+// The persistent kernel takes light tiles (the bins of the raster queue below the heavy classes,
+// heaviest class first) from their own counter, then helps clear the bins without entries. k_raster takes the heavy tiles.
 
 constexpr int kWarpUnitWarps = 4;  // warps (independent tiles) per CTA of k_raster_warp
 // CTAs per SM the launch bounds aim at: with 4 samples the shared sample tiles allow 5; with
@@ -37,6 +36,7 @@ struct alignas(16) WarpUnitSmem {
 
 template <int S, int TS>
 struct WarpRasterSmem {
+    TileQueue tq;
     WarpUnitSmem<S, TS> u[kWarpUnitWarps];
 };
 
@@ -510,14 +510,14 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const FrameDe
 }
 
 // Persistent warp-per-tile raster kernel over the light tiles of one raster launch: the bins
-// order[nheavy .. nbusy) (queue[3] = nheavy, queue[2] = nbusy, both written by k_tile_order),
-// times nsx * nsx quadrants, taken one tile per warp from queue[4]; then bins without entries
-// from queue[1], like k_raster.
+// past the heavy classes, times nsx * nsx quadrants, taken one tile per warp from queue[2]; then bins
+// without entries from queue[1], like k_raster.
 template <int S, int TS>
 __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 : kWarpUnitCtas) k_raster_warp(const FrameDev* __restrict__ frames,
                                                                      int nframes,
                                                                      const uint32_t* __restrict__ order,
-                                                                     uint32_t ntotal, uint32_t nsx,
+                                                                     uint32_t ntotal, uint32_t first_tile,
+                                                                     uint32_t nsx,
                                                                      unsigned int* __restrict__ queue,
                                                                      const DrawDev* __restrict__ draws,
                                                                      Scratch s) {
@@ -526,17 +526,17 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 :
     WarpRasterSmem<S, TS>& sh = *reinterpret_cast<WarpRasterSmem<S, TS>*>(smem_raw);
     const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
     WarpUnitSmem<S, TS>& sm = sh.u[warp];
-    const uint32_t nbusy = *(volatile unsigned int*)&queue[2];
-    const uint32_t nheavy = *(volatile unsigned int*)&queue[3];
+    load_queue(sh.tq, queue, order, ntotal, s.status, first_tile);
+    const uint32_t nheavy = heavy_tiles(sh.tq, frames[0].heavy_bits);
     const uint32_t nsub = nsx * nsx;
-    const uint32_t nlight = (nbusy - nheavy) * nsub;
+    const uint32_t nlight = (sh.tq.busy - nheavy) * nsub;
     uint32_t shaded = 0, fsinv = 0, oobc = 0;
     for (;;) {
         uint32_t qi = 0;
-        if (lane == 0) qi = atomicAdd(&queue[4], 1u);
+        if (lane == 0) qi = atomicAdd(&queue[2], 1u);
         qi = __shfl_sync(0xFFFFFFFFu, qi, 0);
         if (qi >= nlight) break;
-        const uint32_t gt = order[nheavy + qi / nsub], sub = qi % nsub;
+        const uint32_t gt = busy_tile(sh.tq, nheavy + qi / nsub), sub = qi % nsub;
         const FrameDev& f = frames[frame_of_tile(frames, nframes, gt)];
         const uint32_t lt = gt - f.tile_begin;
         const uint32_t X0 = (lt % f.tiles_x) * (uint32_t)f.ts + (sub % nsx) * TS;
@@ -556,11 +556,11 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 :
     for (;;) {
         uint32_t q0 = 0;
         if (lane == 0) q0 = atomicAdd(&queue[1], (unsigned)kEmptyRun);
-        q0 = __shfl_sync(0xFFFFFFFFu, q0, 0) + nbusy;
-        if (q0 >= ntotal) break;
-        const uint32_t q1 = min(q0 + (uint32_t)kEmptyRun, ntotal);
+        q0 = __shfl_sync(0xFFFFFFFFu, q0, 0);
+        if (q0 >= sh.tq.empty) break;
+        const uint32_t q1 = min(q0 + (uint32_t)kEmptyRun, sh.tq.empty);
         for (uint32_t qi = q0; qi < q1; ++qi) {
-            const uint32_t gt = order[qi];
+            const uint32_t gt = empty_tile(sh.tq, qi);
             const FrameDev& f = frames[frame_of_tile(frames, nframes, gt)];
             const uint32_t lt = gt - f.tile_begin;
             const uint32_t edge = (uint32_t)f.ts;

@@ -54,7 +54,6 @@ struct Slot {
     std::vector<uint64_t> ids;
     std::vector<FrameJob> jobs;
     uint64_t bytes = 0;
-    HostBuf<unsigned long long> need;
     void* server = nullptr;
 };
 
@@ -186,11 +185,9 @@ struct rast_server {
         sl.E.sync_after = false;
         rast_status st = run_frames(sl.E, sl.jobs);
         const size_t nf = sl.jobs.size();
-        bool ok = st == RAST_OK && sl.need.reserve(nf);
+        bool ok = st == RAST_OK;
         if (ok) {
-            cudaMemcpyAsync(sl.E.h_state, sl.E.d_state, sizeof(DeviceState), cudaMemcpyDeviceToHost, sl.E.stream);
-            cudaMemcpyAsync(sl.need.p, sl.E.frame_need.p, nf * sizeof(unsigned long long),
-                            cudaMemcpyDeviceToHost, sl.E.stream);
+            cudaMemcpyAsync(sl.E.h_state, sl.E.d_state, Engine::state_bytes(nf), cudaMemcpyDeviceToHost, sl.E.stream);
             ok = cudaLaunchHostFunc(sl.E.stream, on_slot_done, &sl) == cudaSuccess;
         }
         lk.lock();
@@ -223,7 +220,7 @@ struct rast_server {
             const FrameJob& J = sl.jobs[sl.E.h_order[k]];
             const rast_scene& s = reqs[sl.ids[sl.E.h_order[k]]].scene;
             uint64_t& h = bins_hint[ShapeKey{s.mesh, s.width, s.height, s.msaa, J.ts}];
-            h = std::max<uint64_t>(h, sl.need.p[k] + sl.need.p[k] / 8 + 1024);
+            h = std::max<uint64_t>(h, sl.E.h_need()[k] + sl.E.h_need()[k] / 8 + 1024);
         }
         if (status & ST_CLIP_STORE_OVERFLOW)
             sl.E.clip_hint = sl.E.h_state->clip_used + sl.E.h_state->clip_used / 4 + 65536;

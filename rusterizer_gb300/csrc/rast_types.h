@@ -35,9 +35,14 @@ constexpr unsigned long long kRectEmpty = ~0ull;
 // band of kCountBandTiles bins, so the automatic bin size avoids them where it can
 constexpr int kCountBandTiles = 16384;
 constexpr int kMaxTilesPerFrame = 1 << 22;
-// Raster tile queue counters per (msaa, tile) launch group: [0] heavy-tile tickets, [1] empty-bin
-// tickets, [2] bins with entries, [3] heavy bins, [4] light-tile tickets
-constexpr int kQueueSlots = 8;
+// Raster tile queue of one (msaa, tile) launch group: counters [0] heavy-tile tickets, [1] empty-bin
+// tickets, [2] light-tile tickets, [4 + c] bins of class c. Classes order the bins roughly heaviest
+// first (0: no entries; see order_class); the bins of each class are listed by the kernel that
+// counts them, in no particular order, at order_slot.
+constexpr int kQueueSlots = 16;
+constexpr int kQueueClass = 4;
+constexpr int kClasses = 12;
+constexpr int kOrderArrays = kClasses / 2;  // arrays of tiles per raster group
 constexpr int kMaxRasterGroups = 8;
 // Bins with at least 2^kDefaultHeavyBits entries are rastered CTA-wide, the others one warp per
 // raster tile (rast_set_heavy_tile_entries)
@@ -121,6 +126,11 @@ struct FrameDev {
     unsigned long long bin_base;    // offset of this frame's bins
     unsigned long long bin_cap;     // bins reserved for this frame
     unsigned long long qbin_base;   // offset of this frame's quadrant lists (32-pixel bins)
+    uint32_t queue;        // raster group (its counters: Scratch::queues + kQueueSlots * queue)
+    uint32_t order_begin;  // the group's first tile; its lists start at kOrderArrays * order_begin
+    uint32_t order_n;      // tiles of the group
+    uint32_t heavy_bits;   // bins of >= 2^heavy_bits entries are rastered CTA-wide (32: none)
+    uint32_t order_coarse; // only classes 0 and 1 are used: the group's lists need one array
     float clear_depth;
     uint32_t* out;         // width * height ARGB (device)
     float* dbg_depth;      // optional [y][x][s]
@@ -143,7 +153,8 @@ struct Scratch {
     uint32_t* counts;
     uint32_t* tile_start;
     uint32_t* tile_count;
-    uint32_t* tile_order;               // raster queue: tiles by decreasing entry count
+    uint32_t* tile_order;               // raster queues: kOrderArrays arrays of tiles per raster group
+    unsigned int* queues;               // raster queue counters
     uint32_t* bins;
     uint32_t* qbins;                    // per 32-pixel bin: its entries split by raster quadrant
     uint32_t* qcount;                   // [4 * tile + quadrant] entries in each quadrant list
@@ -155,7 +166,7 @@ struct Scratch {
     unsigned long long* clip_used;      // floats allocated this frame
     uint32_t* status;
     unsigned long long* stats;          // StatSlots
-    unsigned long long* frame_need;     // per frame: bin entries needed
+    unsigned long long* frame_need;     // per frame: bin entries allocated so far, then needed
     uint32_t* log;
     unsigned long long* log_n;
     unsigned long long log_cap;
