@@ -73,6 +73,13 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         return jobs[a].ts < jobs[b].ts;
     });
     E.h_order = order;
+    // every frame small: the front and gather kernels (see k_bin_gather)
+    bool small = true;
+    for (const FrameJob& J : jobs) {
+        uint64_t t = 0;
+        for (const DrawJob& DJ : J.draws) t += DJ.mesh->ntris;
+        small = small && t <= kGatherTris;
+    }
 
     for (int attempt = 0; attempt < 3; ++attempt) {
         std::vector<FrameDev>& frames = E.h_frames;
@@ -124,7 +131,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
                 const uint32_t di = (uint32_t)draws.size();
                 draws.push_back(D);
                 for (uint32_t v = 0; v < m->nverts; v += 256) vblocks.push_back(make_uint2(di, v));
-                const uint32_t cs = chunk_size_for(std::max<uint32_t>(J.ntris_hint, m->ntris));
+                const uint32_t cs = small ? kGatherChunk : chunk_size_for(std::max<uint32_t>(J.ntris_hint, m->ntris));
                 for (uint32_t t = 0; t < m->ntris; t += cs) {
                     ChunkDev C{};
                     C.draw = di;
@@ -146,10 +153,11 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
             F.qbin_base = qbin_tot;
             if (raster_edge(J.ts) < J.ts) qbin_tot += 4ull * want;
             clip_est += 32ull * tb + 4096ull;
-            count_tot += (uint64_t)F.nchunks * F.ntiles;
+            if (!small) count_tot += (uint64_t)F.nchunks * F.ntiles;
             ttot += tb;
             tile_tot += F.ntiles;
-            group_tot += (F.ntiles + 31) / 32;
+            F.gather_bins = gather_edge(F.tiles_x, F.tiles_y);
+            group_tot += small ? gather_groups(F.tiles_x, F.tiles_y, F.gather_bins) : (F.ntiles + 31) / 32;
             max_tiles = std::max(max_tiles, F.ntiles);
             frames.push_back(F);
         }
@@ -171,11 +179,11 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
             i = j;
         }
         // scratch
-        bool ok = E.vclip.reserve(vtot) && E.vscr.reserve(vtot) && E.vcode.reserve(vtot) &&
+        bool ok = E.vclip.reserve(small ? 0 : vtot) && E.vscr.reserve(vtot) && E.vcode.reserve(small ? 0 : vtot) &&
                   E.tri_rect.reserve(ttot) && E.tri_aux.reserve(ttot) &&
                   E.counts.reserve(count_tot) && E.tile_start.reserve(tile_tot) &&
                   E.tile_count.reserve(tile_tot) && E.tile_order.reserve((uint64_t)kOrderArrays * tile_tot) &&
-                  E.bins.reserve(bin_tot) && E.qbins.reserve(qbin_tot) && E.clip_list.reserve(3ull * ttot) &&
+                  E.bins.reserve(bin_tot) && E.qbins.reserve(qbin_tot) && E.clip_list.reserve(small ? 0 : 3ull * ttot) &&
                   E.qcount.reserve(qbin_tot ? 4ull * tile_tot : 0ull) &&
                   E.clip_store.reserve(std::max<uint64_t>(clip_est, E.clip_hint)) &&
                   E.reserve_state(frames.size());
@@ -253,13 +261,13 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
 
         cudaError_t err = cudaSuccess;
         if (E.profiling) cudaEventRecord(E.ev[0], st);
-        err = launch_vertex(a);
+        err = small ? launch_front(a) : launch_vertex(a);
         if (E.profiling) cudaEventRecord(E.ev[1], st);
-        if (err == cudaSuccess) err = launch_bin_count(a);
+        if (err == cudaSuccess && !small) err = launch_bin_count(a);
         if (E.profiling) cudaEventRecord(E.ev[2], st);
-        if (err == cudaSuccess) err = launch_scans(a);
+        if (err == cudaSuccess && !small) err = launch_scans(a);
         if (E.profiling) cudaEventRecord(E.ev[3], st);
-        if (err == cudaSuccess) err = launch_bin_scatter(a);
+        if (err == cudaSuccess) err = small ? launch_gather(a) : launch_bin_scatter(a);
         if (E.profiling) cudaEventRecord(E.ev[4], st);
         // raster: one launch per (msaa, tile) group of consecutive frames; with several groups
         // (batches of mixed MSAA) they alternate between the context stream and its side stream,

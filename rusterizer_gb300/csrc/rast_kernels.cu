@@ -7,6 +7,7 @@
 //   k_scan_cols    per tile: exclusive prefix of the histograms over chunks; per 32 tiles: their bin
 //                  ranges, capacity check, and their places in the raster tile queue
 //   k_bin_scatter  per chunk: order-preserving scatter of triangle ids into tile bins
+//   k_front, k_bin_gather   in place of all these when every frame is small
 //   k_bin_split    per 32-pixel bin: its entries split into four 16-pixel quadrant lists
 //   k_raster<S,TS> per raster tile, a CTA of 4 warps: replays the tile's triangles in
 //                  submission order with all colour/depth samples in shared memory; coverage,
@@ -120,6 +121,14 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* tmp, u
 }
 
 // ===================================================================== vertex stage
+
+// vertex shader P*V*W*v (upstream src/main.rs:147-152) with MVP folded on the host in the
+// same dot order; Mat4 * Vec4 is src/math/vector.rs:219-240
+__device__ __forceinline__ float4 vertex_clip(const DrawDev& d, uint32_t v) {
+    const float x = __ldg(d.pos + 3ull * v), y = __ldg(d.pos + 3ull * v + 1), z = __ldg(d.pos + 3ull * v + 2);
+    return make_float4(dot4(d.mvp + 0, x, y, z, 1.0f), dot4(d.mvp + 4, x, y, z, 1.0f),
+                       dot4(d.mvp + 8, x, y, z, 1.0f), dot4(d.mvp + 12, x, y, z, 1.0f));
+}
 
 __global__ void __launch_bounds__(256) k_vertex(const DrawDev* __restrict__ draws,
                                                 const FrameDev* __restrict__ frames,
@@ -249,11 +258,86 @@ __device__ __forceinline__ int warp_clip(ClipVert& v, int cn) {
     return cn;
 }
 
-// Clips the queued straddling triangles, one warp per triangle: the polygon goes to the clip
-// store in screen space (to_screen per vertex, as the reference divides and maps the fan's
-// triangles, src/rasterizer/mod.rs:425-441), the union of the fan's pixel boxes
-// (clipping.rs:185-190) becomes the triangle's box, and its tiles are added to its chunk's
-// counts. Grid-stride over the queue.
+// Clips one straddling triangle with a whole warp: lane q < 3 holds vertex index vi and clip-space
+// position c of corner q. The polygon goes to the clip store in screen space (to_screen per vertex, as
+// the reference divides and maps the fan's triangles, src/rasterizer/mod.rs:425-441); the union
+// of the fan's pixel boxes (clipping.rs:185-190) is the triangle's box. Returns the box
+// (kRectEmpty when nothing can be covered) and the polygon's offset, the same in every lane.
+__device__ __forceinline__ unsigned long long clip_triangle(const DrawDev& d, const FrameDev& f, const Scratch& s,
+                                                            uint32_t vi, float4 c, uint32_t& off32) {
+    const uint32_t lane = lane_id();
+    ClipVert v;
+    if (lane < 3) {
+        v.p[0] = c.x;
+        v.p[1] = c.y;
+        v.p[2] = c.z;
+        v.p[3] = c.w;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v.a[q] = d.rgba ? __ldg(d.rgba + 4ull * vi + q) : 0.0f;
+        v.a[4] = __ldg(d.uv + 2ull * vi);
+        v.a[5] = __ldg(d.uv + 2ull * vi + 1);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v.p[k] = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) v.a[k] = 0.0f;
+    }
+    const int n = warp_clip(v, 3);
+    if (n < 0) {
+        if (lane == 0) atomicOr(s.status, ST_CLIP_OVERFLOW);
+        return kRectEmpty;
+    }
+    if (n < 3) return kRectEmpty;
+    const unsigned long long need = 1ull + 10ull * (unsigned long long)n;
+    unsigned long long off = 0;
+    if (lane == 0) off = atomicAdd(s.clip_used, need);
+    off = __shfl_sync(0xFFFFFFFFu, off, 0);
+    if (off + need > s.clip_cap) {
+        if (lane == 0) atomicOr(s.status, ST_CLIP_STORE_OVERFLOW);
+        return kRectEmpty;
+    }
+    float* st = s.clip_store + off;
+    const float4 sc = to_screen(make_float4(v.p[0], v.p[1], v.p[2], v.p[3]), (float)f.width, (float)f.height);
+    if (lane == 0) st[0] = __int_as_float(n);
+    if (lane < (uint32_t)n) {
+        float* o = st + 1 + 10 * lane;
+        o[0] = sc.x;
+        o[1] = sc.y;
+        o[2] = sc.z;
+        o[3] = sc.w;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) o[4 + q] = v.a[q];
+    }
+    // fan triangle `lane`: vertices 0, lane + 1, lane + 2
+    float4 tv[3];
+    tv[0] = make_float4(__shfl_sync(0xFFFFFFFFu, sc.x, 0), __shfl_sync(0xFFFFFFFFu, sc.y, 0),
+                        __shfl_sync(0xFFFFFFFFu, sc.z, 0), __shfl_sync(0xFFFFFFFFu, sc.w, 0));
+    const uint32_t l1 = min(lane + 1, 31u), l2 = min(lane + 2, 31u);
+    tv[1] = make_float4(__shfl_sync(0xFFFFFFFFu, sc.x, l1), __shfl_sync(0xFFFFFFFFu, sc.y, l1),
+                        __shfl_sync(0xFFFFFFFFu, sc.z, l1), __shfl_sync(0xFFFFFFFFu, sc.w, l1));
+    tv[2] = make_float4(__shfl_sync(0xFFFFFFFFu, sc.x, l2), __shfl_sync(0xFFFFFFFFu, sc.y, l2),
+                        __shfl_sync(0xFFFFFFFFu, sc.z, l2), __shfl_sync(0xFFFFFFFFu, sc.w, l2));
+    uint32_t a0 = 0xFFFFFFFFu, a1 = 0, b0 = 0xFFFFFFFFu, b1 = 0;
+    if (lane + 2 < (uint32_t)n) {
+        uint32_t x0, x1, y0, y1;
+        pixel_bbox(tv, f.width, f.height, x0, x1, y0, y1);
+        if (x0 < x1 && y0 < y1) {
+            a0 = x0;
+            a1 = x1;
+            b0 = y0;
+            b1 = y1;
+        }
+    }
+    a0 = __reduce_min_sync(0xFFFFFFFFu, a0);
+    a1 = __reduce_max_sync(0xFFFFFFFFu, a1);
+    b0 = __reduce_min_sync(0xFFFFFFFFu, b0);
+    b1 = __reduce_max_sync(0xFFFFFFFFu, b1);
+    off32 = (uint32_t)off;
+    return a0 < a1 && b0 < b1 ? pack_rect(a0, b0, a1 - 1, b1 - 1) : kRectEmpty;
+}
+
+// Clips the queued straddling triangles, one warp per triangle (grid-stride over the queue), and
+// adds their tiles to their chunks' counts.
 __global__ void __launch_bounds__(256) k_clip(const DrawDev* __restrict__ draws,
                                               const FrameDev* __restrict__ frames, Scratch s) {
     pdl_enter();
@@ -264,80 +348,18 @@ __global__ void __launch_bounds__(256) k_clip(const DrawDev* __restrict__ draws,
         const uint32_t di = s.clip_list[3ull * e], tri = s.clip_list[3ull * e + 1], row = s.clip_list[3ull * e + 2];
         const DrawDev& d = draws[di];
         const FrameDev& f = frames[d.frame];
-        ClipVert v;
+        uint32_t vi = 0, off = 0;
+        float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (lane < 3) {
-            const uint32_t vi = __ldg(d.idx + 3ull * tri + lane);
-            const float4 c = s.vclip[d.vbase + vi];
-            v.p[0] = c.x;
-            v.p[1] = c.y;
-            v.p[2] = c.z;
-            v.p[3] = c.w;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) v.a[q] = d.rgba ? __ldg(d.rgba + 4ull * vi + q) : 0.0f;
-            v.a[4] = __ldg(d.uv + 2ull * vi);
-            v.a[5] = __ldg(d.uv + 2ull * vi + 1);
-        } else {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) v.p[k] = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 6; ++k) v.a[k] = 0.0f;
+            vi = __ldg(d.idx + 3ull * tri + lane);
+            c = s.vclip[d.vbase + vi];
         }
-        const int n = warp_clip(v, 3);
-        if (n < 0) {
-            if (lane == 0) atomicOr(s.status, ST_CLIP_OVERFLOW);
-            continue;
-        }
-        if (n < 3) continue;
-        const unsigned long long need = 1ull + 10ull * (unsigned long long)n;
-        unsigned long long off = 0;
-        if (lane == 0) off = atomicAdd(s.clip_used, need);
-        off = __shfl_sync(0xFFFFFFFFu, off, 0);
-        if (off + need > s.clip_cap) {
-            if (lane == 0) atomicOr(s.status, ST_CLIP_STORE_OVERFLOW);
-            continue;
-        }
-        float* st = s.clip_store + off;
-        const float4 sc = to_screen(make_float4(v.p[0], v.p[1], v.p[2], v.p[3]), (float)f.width, (float)f.height);
-        if (lane == 0) st[0] = __int_as_float(n);
-        if (lane < (uint32_t)n) {
-            float* o = st + 1 + 10 * lane;
-            o[0] = sc.x;
-            o[1] = sc.y;
-            o[2] = sc.z;
-            o[3] = sc.w;
-#pragma unroll
-            for (int q = 0; q < 6; ++q) o[4 + q] = v.a[q];
-        }
-        // fan triangle `lane`: vertices 0, lane + 1, lane + 2
-        float4 tv[3];
-        tv[0] = make_float4(__shfl_sync(0xFFFFFFFFu, sc.x, 0), __shfl_sync(0xFFFFFFFFu, sc.y, 0),
-                            __shfl_sync(0xFFFFFFFFu, sc.z, 0), __shfl_sync(0xFFFFFFFFu, sc.w, 0));
-        const uint32_t l1 = min(lane + 1, 31u), l2 = min(lane + 2, 31u);
-        tv[1] = make_float4(__shfl_sync(0xFFFFFFFFu, sc.x, l1), __shfl_sync(0xFFFFFFFFu, sc.y, l1),
-                            __shfl_sync(0xFFFFFFFFu, sc.z, l1), __shfl_sync(0xFFFFFFFFu, sc.w, l1));
-        tv[2] = make_float4(__shfl_sync(0xFFFFFFFFu, sc.x, l2), __shfl_sync(0xFFFFFFFFu, sc.y, l2),
-                            __shfl_sync(0xFFFFFFFFu, sc.z, l2), __shfl_sync(0xFFFFFFFFu, sc.w, l2));
-        uint32_t a0 = 0xFFFFFFFFu, a1 = 0, b0 = 0xFFFFFFFFu, b1 = 0;
-        if (lane + 2 < (uint32_t)n) {
-            uint32_t x0, x1, y0, y1;
-            pixel_bbox(tv, f.width, f.height, x0, x1, y0, y1);
-            if (x0 < x1 && y0 < y1) {
-                a0 = x0;
-                a1 = x1;
-                b0 = y0;
-                b1 = y1;
-            }
-        }
-        a0 = __reduce_min_sync(0xFFFFFFFFu, a0);
-        a1 = __reduce_max_sync(0xFFFFFFFFu, a1);
-        b0 = __reduce_min_sync(0xFFFFFFFFu, b0);
-        b1 = __reduce_max_sync(0xFFFFFFFFu, b1);
-        if (a0 >= a1 || b0 >= b1) continue;
-        const unsigned long long rect = pack_rect(a0, b0, a1 - 1, b1 - 1);
+        const unsigned long long rect = clip_triangle(d, f, s, vi, c, off);
+        if (rect == kRectEmpty) continue;
         const uint32_t g = f.rect_base + d.tbase + tri;
         if (lane == 0) {
-            s.tri_rect[g] = rect;
-            s.tri_aux[g] = (uint32_t)off;
+            s.tri_rect[g] = rect | kRectClippedBit;
+            s.tri_aux[g] = off;
         }
         uint32_t x0, y0, x1, y1;
         tile_rect(rect, (uint32_t)f.ts, x0, y0, x1, y1);
@@ -433,12 +455,13 @@ __device__ __forceinline__ unsigned long long order_slot(uint32_t c, uint32_t k,
     return (unsigned long long)(c >> 1) * n + ((c & 1u) ? k : n - 1 - k);
 }
 
-// Called by one warp whose lane holds bin t of frame f (live lanes) and its entry count: allocates
+// Called by one warp whose lane holds bin t of frame f (live lanes) and its entry count; returns the
+// bin's first entry. Allocates
 // the bins' ranges in one step (the ranges of a frame lie in no particular order), checks the
 // capacity and lists the bins in the raster queue. A prefix over a frame's tiles and a sort
 // of them took two one-CTA kernels before (2M-triangle 4K terrain 13 us, 20 scenes 54 us).
-__device__ __forceinline__ void place_bins(const FrameDev& f, uint32_t frame, const Scratch& s, uint32_t t, bool live,
-                                           uint32_t count) {
+__device__ __forceinline__ uint32_t place_bins(const FrameDev& f, uint32_t frame, const Scratch& s, uint32_t t,
+                                               bool live, uint32_t count) {
     const uint32_t lane = lane_id();
     uint32_t incl = live ? count : 0u;
 #pragma unroll
@@ -466,6 +489,7 @@ __device__ __forceinline__ void place_bins(const FrameDev& f, uint32_t frame, co
         s.tile_start[gt] = (uint32_t)base + incl - count;
         s.tile_order[(unsigned long long)kOrderArrays * f.order_begin + order_slot(c, slot, f.order_n)] = gt;
     }
+    return (uint32_t)base + incl - count;
 }
 
 // One block per 32-tile group of a frame; 32 segments of chunks per tile: the exclusive prefix of
@@ -529,7 +553,6 @@ constexpr int kPairsPerBatch = 512;  // (triangle, tile) pairs ranked per batch
 constexpr uint32_t kBigTri = 32;     // triangles over more tiles are binned alone, tile-parallel
 constexpr int kHashSlots = 1024;     // open-addressing table over tile ids, load <= 0.5
 constexpr uint32_t kHashEmpty = 0xFFFFFFFFu;
-constexpr unsigned long long kRectClippedBit = 1ull << 63;  // pixel boxes stay below 2^15
 
 __device__ __forceinline__ uint32_t hash_slot(uint32_t t) {
     return (t * 2654435761u) >> (32 - 10);
@@ -590,9 +613,8 @@ __global__ void __launch_bounds__(kScatterThreads) k_bin_scatter(
             const uint32_t i = base + v;
             const bool live = i < ch.tri_count;
             r[j] = live ? s.tri_rect[gbase + i] : kRectEmpty;
-            const bool clipped = live && r[j] != kRectEmpty && s.tri_aux[gbase + i] != kNone;
-            n[j] = rect_tiles(r[j], ts);
-            trect[v] = clipped ? (r[j] | kRectClippedBit) : r[j];
+            n[j] = r[j] == kRectEmpty ? 0u : rect_tiles(r[j] & ~kRectClippedBit, ts);
+            trect[v] = r[j];
             mine += n[j];
         }
         if (threadIdx.x == 0) take_s = kScatterWindow;
@@ -746,6 +768,243 @@ __global__ void __launch_bounds__(kScatterThreads) k_bin_scatter(
         if (threadIdx.x == 0) nslots = 0;
         __syncthreads();
         base += take;
+    }
+}
+
+// ===================================================================== small frames: front, gather
+//
+// Frames of at most kGatherTris triangles (every frame of the run) skip the chunk histograms, the
+// column scan and the scatter: a chunk holds 256 triangles or more, so such a frame has a few chunks
+// and the scatter's CTAs, each serial over its triangles, leave the GPU idle; triangles over many bins
+// make it worse (12 chunks of large triangles at 1440p: 324 us). Here vertices, classification and
+// clipping are one launch over as many warps as there are triangles to clip, and the bins are
+// filled from the tiles' side: each CTA owns a block of bins and looks at every triangle's box.
+// Measured a frame, before -> now: 3 000 triangles of 32-512 pixels at 1440p 822 -> 478 us, four demo
+// objects at 720p 193 -> 57 us, the cube 97 -> 72 us, soups of 1 000 to 8 000 triangles (1-64 pixels) at
+// 640x480 57 -> 38 .. 93 -> 85 us and at 4K 69 -> 55 .. 168 -> 159 us. Beyond 8 160 triangles the boxes
+// no longer fit shared memory, and the chunks begin to fill the GPU (8 000 small terrain triangles
+// on 640x480 are the one case that the chunk path does better: 54 against 60 us).
+
+constexpr int kFrontTris = 4;                            // triangles per warp of k_front
+constexpr int kFrontChunk = 8 * kFrontTris;              // per CTA
+static_assert(kFrontChunk == (int)kGatherChunk, "chunks of small frames are one CTA of k_front");
+
+// The first vertex_blocks CTAs transform 256 vertices each (what the raster reads: screen points); the
+// others take a chunk of kFrontChunk triangles, kFrontTris per warp: lane 3 t + q transforms corner
+// q of triangle t again from its position (no wait for the vertex CTAs), lane t classifies triangle t,
+// and the whole warp clips the ones that straddle a plane, one after another. Few triangles per
+// warp, from as many places of the mesh, keep that chain short: a mesh may hold all its
+// straddlers in a row (2 000 triangles, 200 straddlers: 13 us with four neighbours per warp, 9 spread).
+__global__ void __launch_bounds__(256) k_front(const ChunkDev* __restrict__ chunks,
+                                               const DrawDev* __restrict__ draws,
+                                               const FrameDev* __restrict__ frames,
+                                               const uint2* __restrict__ vblocks, uint32_t vertex_blocks, Scratch s) {
+    pdl_enter();
+    if (blockIdx.x < vertex_blocks) {
+        const uint2 vb = vblocks[blockIdx.x];
+        const DrawDev& d = draws[vb.x];
+        const FrameDev& f = frames[d.frame];
+        const uint32_t v = vb.y + threadIdx.x;
+        if (v >= d.nverts) return;
+        s.vscr[d.vbase + v] = to_screen(vertex_clip(d, v), (float)f.width, (float)f.height);
+        return;
+    }
+    const ChunkDev ch = chunks[blockIdx.x - vertex_blocks];
+    const DrawDev& d = draws[ch.draw];
+    const FrameDev& f = frames[d.frame];
+    const uint32_t lane = lane_id();
+    // triangle t of this warp: tri0 + t * nw, nw warps in the draw
+    const uint32_t nw = (d.ntris + kFrontTris - 1) / kFrontTris;
+    const uint32_t tri0 = ch.tri_begin / kFrontTris + (threadIdx.x >> 5);
+    if (tri0 >= nw) return;  // whole warps
+    const uint32_t nt = min((uint32_t)kFrontTris, (d.ntris - tri0 + nw - 1) / nw);
+    uint32_t vi = 0, code = 0;
+    bool bad = false;
+    float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f), sc = c;
+    if (lane < 3 * nt) {
+        vi = __ldg(d.idx + 3ull * (tri0 + lane / 3 * nw) + lane % 3);
+        bad = vi >= d.nverts;
+        if (!bad) {
+            c = vertex_clip(d, vi);
+            code = clip_code(c);
+            sc = to_screen(c, (float)f.width, (float)f.height);
+        }
+    }
+    const uint32_t bads = __ballot_sync(0xFFFFFFFFu, bad);
+    const uint32_t q0 = min(3 * lane, 29u);  // lane t: its corners are lanes 3 t .. 3 t + 2
+    float cx[3], cy[3];
+    float4 sv[3];
+    uint32_t cd[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        cx[q] = __shfl_sync(0xFFFFFFFFu, c.x, q0 + q);
+        cy[q] = __shfl_sync(0xFFFFFFFFu, c.y, q0 + q);
+        cd[q] = __shfl_sync(0xFFFFFFFFu, code, q0 + q);
+        sv[q] = make_float4(__shfl_sync(0xFFFFFFFFu, sc.x, q0 + q), __shfl_sync(0xFFFFFFFFu, sc.y, q0 + q), 0.0f, 0.0f);
+    }
+    const uint32_t g0 = f.rect_base + d.tbase + tri0;
+    bool straddles = false;
+    if (lane < nt) {
+        unsigned long long rect = kRectEmpty;
+        if ((bads >> (3 * lane)) & 7u) {
+            atomicOr(s.status, ST_BAD_INDEX);  // skipped, as in classify_triangle
+        } else {
+            const int cls = clip_classify(tri2x_area(cx[0], cy[0], cx[1], cy[1], cx[2], cy[2]), cd[0], cd[1], cd[2]);
+            if (cls == 1) {
+                uint32_t x0, x1, y0, y1;
+                pixel_bbox(sv, f.width, f.height, x0, x1, y0, y1);
+                if (x0 < x1 && y0 < y1) rect = pack_rect(x0, y0, x1 - 1, y1 - 1);
+            }
+            straddles = cls == 2;
+        }
+        s.tri_rect[g0 + lane * nw] = rect;
+        s.tri_aux[g0 + lane * nw] = kNone;
+    }
+    for (uint32_t m = __ballot_sync(0xFFFFFFFFu, straddles); m; m &= m - 1) {
+        const uint32_t t = __ffs(m) - 1, src = min(3 * t + lane, 31u);
+        const uint32_t cvi = __shfl_sync(0xFFFFFFFFu, vi, src);
+        const float4 cc = make_float4(__shfl_sync(0xFFFFFFFFu, c.x, src), __shfl_sync(0xFFFFFFFFu, c.y, src),
+                                      __shfl_sync(0xFFFFFFFFu, c.z, src), __shfl_sync(0xFFFFFFFFu, c.w, src));
+        uint32_t off = 0;
+        const unsigned long long rect = clip_triangle(d, f, s, cvi, cc, off);
+        if (rect != kRectEmpty && lane == 0) {
+            s.tri_rect[g0 + t * nw] = rect | kRectClippedBit;
+            s.tri_aux[g0 + t * nw] = off;
+        }
+        __syncwarp();
+    }
+}
+
+constexpr int kGatherThreads = 512;
+constexpr int kGatherWarps = kGatherThreads / 32;
+static_assert(kGatherWarps == 16, "16 warps share the block's 64 or 16 bins");
+static_assert(kGatherTris % 32 == 0 && kGatherTris / 32 < 256, "a lane's entries of a bin fit a byte");
+
+// One CTA per block of B x B bins of a frame, B = 8 or 4 (gather_edge). It lists the triangles whose boxes
+// touch the block (in submission order: every warp a contiguous part of the mesh, two passes), then
+// each warp fills half a row of 8 bins (or one bin of 4 x 4) from the list: one pass counts (byte
+// counters in the lanes), the bins' ranges are allocated (place_bins), a second pass writes each
+// bin's entries in order.
+__global__ void __launch_bounds__(kGatherThreads) k_bin_gather(const FrameDev* __restrict__ frames, int nframes,
+                                                               Scratch s) {
+    pdl_enter();
+    __shared__ uint16_t abox[kGatherTris];  // by triangle: bins of the block x0 | x1 << 3 | y0 << 6 | y1 << 9 | clipped << 15
+    __shared__ uint16_t ltri[kGatherTris];  // the block's triangles in order
+    __shared__ uint32_t hit[kGatherTris / 32];
+    __shared__ uint32_t wcount[kGatherWarps];
+    __shared__ uint32_t bcount[64], bstart[64];
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    int fi = 0;
+    {
+        int hi = nframes;
+        while (hi - fi > 1) {
+            const int mid = (fi + hi) >> 1;
+            if (frames[mid].group_begin <= blockIdx.x) fi = mid; else hi = mid;
+        }
+    }
+    const FrameDev& f = frames[fi];
+    const uint32_t B = f.gather_bins;
+    const uint32_t bx = (f.tiles_x + B - 1) / B;
+    const uint32_t blk = blockIdx.x - f.group_begin;
+    const uint32_t X = (blk % bx) * B, Y = (blk / bx) * B;  // the block's first bin
+    // this warp's bins: nb from column col of row
+    const uint32_t nb = B == 8 ? 4u : 1u, row = B == 8 ? warp >> 1 : warp >> 2, col = B == 8 ? 4 * (warp & 1u) : warp & 3u;
+    const uint32_t T = f.ntris, ts = (uint32_t)f.ts;
+    const uint32_t words = (T + 31) / 32, per = (words + kGatherWarps - 1) / kGatherWarps;
+    const uint32_t w0 = min(words, warp * per), w1 = min(words, w0 + per);
+    // ---- the block's triangles (kAhead boxes in flight per lane)
+    uint32_t n = 0;
+    constexpr uint32_t kAhead = 4;
+    for (uint32_t wa = w0; wa < w1; wa += kAhead) {
+        unsigned long long r[kAhead];
+#pragma unroll
+        for (uint32_t k = 0; k < kAhead; ++k) {
+            const uint32_t i = (wa + k) * 32 + lane;
+            r[k] = wa + k < w1 && i < T ? s.tri_rect[f.rect_base + i] : kRectEmpty;
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kAhead; ++k) {
+            if (wa + k >= w1) break;
+            uint32_t x0, y0, x1, y1;
+            tile_rect(r[k] & ~kRectClippedBit, ts, x0, y0, x1, y1);
+            const bool in = r[k] != kRectEmpty && x0 < X + B && x1 >= X && y0 < Y + B && y1 >= Y;
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, in);
+            if (in)
+                abox[(wa + k) * 32 + lane] =
+                    (uint16_t)((max(x0, X) - X) | (min(x1 - X, B - 1) << 3) |
+                               ((max(y0, Y) - Y) << 6) | (min(y1 - Y, B - 1) << 9) |
+                               ((r[k] & kRectClippedBit) ? 0x8000u : 0u));
+            if (lane == 0) hit[wa + k] = m;
+            n += __popc(m);
+        }
+    }
+    if (lane == 0) wcount[warp] = n;
+    __syncthreads();
+    uint32_t at = 0, total = 0;
+#pragma unroll
+    for (int k = 0; k < kGatherWarps; ++k) {
+        const uint32_t c = wcount[k];
+        if ((uint32_t)k < warp) at += c;
+        total += c;
+    }
+    for (uint32_t w = w0; w < w1; ++w) {
+        const uint32_t m = hit[w];
+        if ((m >> lane) & 1u) {
+            const uint32_t i = w * 32 + lane, k = at + __popc(m & lanemask_lt());
+            ltri[k] = (uint16_t)i;
+        }
+        at += __popc(m);
+    }
+    __syncthreads();
+    // ---- entries per bin of the warp: bit k of the mask is bin k
+    auto row_mask = [&](uint32_t b) {
+        const uint32_t x0 = b & 7u, x1 = (b >> 3) & 7u, y0 = (b >> 6) & 7u, y1 = (b >> 9) & 7u;
+        return row >= y0 && row <= y1 ? (((2u << x1) - (1u << x0)) >> col) & ((1u << nb) - 1u) : 0u;
+    };
+    uint32_t counts = 0;  // byte counters of the bins
+    for (uint32_t i = lane; i < total; i += 32) {
+        const uint32_t m = row_mask(abox[ltri[i]]);
+        counts += (m * 0x00204081u) & 0x01010101u;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        if ((uint32_t)k >= nb) break;
+        const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, (counts >> (8 * k)) & 0xFFu);
+        if (lane == 0) bcount[row * B + col + k] = c;
+    }
+    __syncthreads();
+    if (warp * 32 < B * B) {
+        const uint32_t b = warp * 32 + lane, x = X + b % B, y = Y + b / B;
+        const bool live = b < B * B && x < f.tiles_x && y < f.tiles_y;
+        bstart[b] = place_bins(f, (uint32_t)fi, s, y * f.tiles_x + x, live, live ? bcount[b] : 0u);
+    }
+    __syncthreads();
+    // ---- the entries, in order
+    uint32_t* bins = s.bins + f.bin_base;
+    uint32_t pos = lane < nb ? bstart[row * B + col + lane] : 0u;  // lane k: next entry of bin k
+    for (uint32_t i0 = 0; i0 < total; i0 += 32) {
+        const uint32_t i = i0 + lane;
+        uint32_t tri = 0, b = 0x40u;  // (an empty box: rows 1 .. 0)
+        if (i < total) {
+            tri = ltri[i];
+            b = abox[tri];
+        }
+        const uint32_t m = row_mask(b);
+        if (!__any_sync(0xFFFFFFFFu, m != 0)) continue;
+        const bool clipped = (b & 0x8000u) != 0;
+        unsigned long long r = 0;
+        if (m) {
+            if (raster_edge((int)ts) != (int)ts) r = s.tri_rect[f.rect_base + tri] & ~kRectClippedBit;  // its quadrants
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if ((uint32_t)k >= nb) break;
+            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, (m >> k) & 1u);
+            const uint32_t p = __shfl_sync(0xFFFFFFFFu, pos, k) + __popc(bal & lanemask_lt());
+            if (((m >> k) & 1u) && p < f.bin_cap) bins[p] = bin_entry(tri, clipped, r, X + col + k, Y + row, ts);
+            if (lane == (uint32_t)k) pos += __popc(bal);
+        }
     }
 }
 
@@ -1804,6 +2063,17 @@ static cudaError_t launch_raster_t(const LaunchArgs& a, uint32_t nsx) {
 cudaError_t launch_vertex(const LaunchArgs& a) {
     if (a.vertex_blocks == 0) return cudaSuccess;
     return launch_pdl(k_vertex, a.vertex_blocks, 256, 0, a.stream, a.draws, a.frames, a.vblocks, a.scratch);
+}
+
+cudaError_t launch_front(const LaunchArgs& a) {
+    if (a.vertex_blocks + a.nchunks == 0) return cudaSuccess;
+    return launch_pdl(k_front, a.vertex_blocks + a.nchunks, 256, 0, a.stream, a.chunks, a.draws, a.frames, a.vblocks,
+                      a.vertex_blocks, a.scratch);
+}
+
+cudaError_t launch_gather(const LaunchArgs& a) {
+    if (a.scan_groups == 0) return cudaSuccess;
+    return launch_pdl(k_bin_gather, a.scan_groups, kGatherThreads, 0, a.stream, a.frames, a.nframes, a.scratch);
 }
 
 cudaError_t launch_bin_count(const LaunchArgs& a) {

@@ -18,7 +18,7 @@ struct LaunchArgs {
     uint32_t nchunks;
     const uint2* vblocks;  // (draw, first vertex) per 256-vertex block
     uint32_t vertex_blocks;
-    uint32_t scan_groups;  // 32-tile groups over all frames
+    uint32_t scan_groups;  // scan groups over all frames
     uint32_t max_tiles;    // largest per-frame tile count
     // raster launch over one (msaa, tile) group of consecutive frames
     const FrameDev* raster_frames;
@@ -31,6 +31,9 @@ struct LaunchArgs {
     Scratch scratch;
 };
 
+// small runs: launch_front and launch_gather instead of launch_vertex .. launch_bin_scatter
+cudaError_t launch_front(const LaunchArgs& a);
+cudaError_t launch_gather(const LaunchArgs& a);
 cudaError_t launch_vertex(const LaunchArgs& a);
 cudaError_t launch_bin_count(const LaunchArgs& a);
 cudaError_t launch_scans(const LaunchArgs& a);

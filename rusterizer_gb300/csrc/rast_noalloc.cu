@@ -82,7 +82,7 @@ struct Layout {
         torder, bins, qbins, qcount, clip, clist, end;
 };
 
-Layout carve_layout(uint32_t nverts, uint32_t ntris, uint32_t nchunks, uint32_t nvb, uint32_t ntiles,
+Layout carve_layout(uint32_t nverts, uint32_t ntris, uint32_t nchunks, uint32_t count_chunks, uint32_t nvb, uint32_t ntiles,
                     bool split, unsigned long long bin_cap, unsigned long long clip_floats,
                     bool coarse) {
     using namespace rast;
@@ -98,7 +98,7 @@ Layout carve_layout(uint32_t nverts, uint32_t ntris, uint32_t nchunks, uint32_t 
     L.vcode = c.take(sizeof(uint16_t) * (size_t)nverts);
     L.rect = c.take(sizeof(unsigned long long) * (size_t)ntris);
     L.aux = c.take(sizeof(uint32_t) * (size_t)ntris);
-    L.counts = c.take(sizeof(uint32_t) * (size_t)nchunks * ntiles);
+    L.counts = c.take(sizeof(uint32_t) * (size_t)count_chunks * ntiles);
     L.tstart = c.take(sizeof(uint32_t) * ntiles);
     L.tcount = c.take(sizeof(uint32_t) * ntiles);
     L.torder = c.take((coarse ? 1 : kOrderArrays) * sizeof(uint32_t) * (size_t)ntiles);
@@ -141,11 +141,13 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
     if (!ts) return RAST_INVALID_ARG;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    const uint32_t cs = chunk_size_for(ntris);
-    const uint32_t nchunks = (ntris + cs - 1) / cs;
+    const uint32_t big_cs = chunk_size_for(ntris);
+    const uint32_t big_chunks = (ntris + big_cs - 1) / big_cs;
     const uint32_t nvb = (nverts + 255u) / 256u;
     // chunk_size_for never goes below kMinChunk, so the descriptor arrays always hold them
-    if (cs < kMinChunk || nchunks > sizeof(g_chunks) / sizeof(g_chunks[0]) ||
+    static_assert((kGatherTris + kGatherChunk - 1) / kGatherChunk <= sizeof(g_chunks) / sizeof(g_chunks[0]),
+                  "the staging array holds a small frame's chunks");
+    if (big_cs < kMinChunk || big_chunks > sizeof(g_chunks) / sizeof(g_chunks[0]) ||
         nvb > sizeof(g_vblocks) / sizeof(g_vblocks[0]))
         return RAST_INVALID_ARG;
     FrameDev F{};
@@ -159,10 +161,10 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
     F.draw_begin = 0;
     F.draw_count = 1;
     F.ntris = ntris;
-    F.nchunks = nchunks;
     F.clear_depth = clear_depth;
     F.order_n = F.ntiles;
     F.heavy_bits = kDefaultHeavyBits;
+    F.gather_bins = gather_edge(F.tiles_x, F.tiles_y);
     F.out = d_argb;
     DrawDev D{};
     D.pos = d_pos;
@@ -192,12 +194,20 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
     unsigned long long clip_floats = 32ull * ntris + 4096ull;
     for (int attempt = 0; attempt < 3; ++attempt) {
         // the raster queue's lists take kOrderArrays arrays, or one where the rest leaves no room for them
+        // (and a small frame's finer chunks more descriptors); a frame that fits without them takes
+        // the general path
         F.order_coarse = 0;
-        Layout L = carve_layout(nverts, ntris, nchunks, nvb, F.ntiles, split, bin_cap, clip_floats, false);
+        bool small = ntris <= kGatherTris;
+        uint32_t cs = small ? kGatherChunk : big_cs, nchunks = (ntris + cs - 1) / cs;
+        Layout L = carve_layout(nverts, ntris, nchunks, big_chunks, nvb, F.ntiles, split, bin_cap, clip_floats, false);
         if (L.end > kNoAllocScratchBytes) {
             F.order_coarse = 1;
-            L = carve_layout(nverts, ntris, nchunks, nvb, F.ntiles, split, bin_cap, clip_floats, true);
+            small = false;
+            cs = big_cs;
+            nchunks = big_chunks;
+            L = carve_layout(nverts, ntris, nchunks, big_chunks, nvb, F.ntiles, split, bin_cap, clip_floats, true);
         }
+        F.nchunks = nchunks;
         if (L.end > kNoAllocScratchBytes) return RAST_INVALID_ARG;
         F.bin_cap = bin_cap;
 
@@ -236,7 +246,7 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
         a.nchunks = nchunks;
         a.vblocks = reinterpret_cast<const uint2*>(base + L.vblocks);
         a.vertex_blocks = nvb;
-        a.scan_groups = (F.ntiles + 31) / 32;
+        a.scan_groups = small ? gather_groups(F.tiles_x, F.tiles_y, F.gather_bins) : (F.ntiles + 31) / 32;
         a.max_tiles = F.ntiles;
         a.raster_frames = a.frames;
         a.raster_nframes = 1;
@@ -271,10 +281,10 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
         S.log_n = &dstate->log_n;
         S.log_cap = 0;
 
-        cudaError_t err = launch_vertex(a);
-        if (err == cudaSuccess) err = launch_bin_count(a);
-        if (err == cudaSuccess) err = launch_scans(a);
-        if (err == cudaSuccess) err = launch_bin_scatter(a);
+        cudaError_t err = small ? launch_front(a) : launch_vertex(a);
+        if (err == cudaSuccess && !small) err = launch_bin_count(a);
+        if (err == cudaSuccess && !small) err = launch_scans(a);
+        if (err == cudaSuccess) err = small ? launch_gather(a) : launch_bin_scatter(a);
         if (err == cudaSuccess) err = launch_bin_split(a, ts);
         if (err == cudaSuccess) err = launch_raster(a, msaa, ts);
         if (err != cudaSuccess) {

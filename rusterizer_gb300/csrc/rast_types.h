@@ -8,7 +8,7 @@
 //   vscr[v]   float4  (screen x, screen y, screen z, w) after divide + viewport
 //   vcode[v]  u16     clip predicates (rast_device.cuh clip_code)
 //   tri_rect[t] u64   pixel box of triangle t (x0,y0,x1,y1 inclusive, 16 bits each),
-//                     kRectEmpty when culled
+//                     kRectEmpty when culled; bit 63: clipped
 //   tri_aux[t]  u32   offset of the clipped polygon in clip_store, kNone when unclipped
 //   clip_list[] u32×3 triangles that straddle a clip plane (draw, triangle, chunk row), clipped
 //                     afterwards by one warp each (k_clip)
@@ -30,6 +30,7 @@ constexpr float kCullEps = 0.000001f;          // src/rasterizer/clipping.rs:12
 constexpr int kMaxPoly = 32;                   // clip polygon capacity (a convex clip needs 9)
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr unsigned long long kRectEmpty = ~0ull;
+constexpr unsigned long long kRectClippedBit = 1ull << 63;  // pixel boxes stay below 2^15
 // bins of one frame: up to kCountBandTiles are counted in one pass over a chunk's triangles
 // (a 32 KB shared histogram); larger frames (any 16384 x 16384 frame fits) take one pass per
 // band of kCountBandTiles bins, so the automatic bin size avoids them where it can
@@ -65,6 +66,19 @@ inline uint32_t chunk_size_for(uint32_t ntris) {
     uint32_t c = (ntris + 899u) / 900u;
     c = (c + 255u) & ~255u;
     return c < 256u ? 256u : (c > 8192u ? 8192u : c);
+}
+
+// Runs whose frames all have at most kGatherTris triangles take k_front and k_bin_gather: chunks of
+// kGatherChunk triangles, scan groups of gather_edge^2 bins.
+constexpr uint32_t kGatherTris = 8160;
+constexpr uint32_t kGatherChunk = 32;
+inline uint32_t gather_groups(uint32_t tiles_x, uint32_t tiles_y, uint32_t edge) {
+    return ((tiles_x + edge - 1) / edge) * ((tiles_y + edge - 1) / edge);
+}
+// Blocks of 8 x 8 bins where there are enough of them for the GPU, else 4 x 4: more CTAs, each with a
+// shorter list.
+inline uint32_t gather_edge(uint32_t tiles_x, uint32_t tiles_y) {
+    return gather_groups(tiles_x, tiles_y, 8) >= 100 ? 8 : 4;
 }
 
 enum StatusBits : uint32_t {
@@ -120,7 +134,7 @@ struct FrameDev {
     uint32_t ntris;
     uint32_t nchunks;
     uint32_t tile_begin;   // global index of this frame's first tile
-    uint32_t group_begin;  // first 32-tile scan group of this frame
+    uint32_t group_begin;  // first scan group of this frame (32 tiles, or gather_bins^2 in a small run)
     uint32_t rect_base;    // global index of this frame's first triangle in tri_rect/tri_aux
     unsigned long long count_base;  // offset of counts[frame]
     unsigned long long bin_base;    // offset of this frame's bins
@@ -130,6 +144,7 @@ struct FrameDev {
     uint32_t order_begin;  // the group's first tile; its lists start at kOrderArrays * order_begin
     uint32_t order_n;      // tiles of the group
     uint32_t heavy_bits;   // bins of >= 2^heavy_bits entries are rastered CTA-wide (32: none)
+    uint32_t gather_bins;  // block edge of k_bin_gather
     uint32_t order_coarse; // only classes 0 and 1 are used: the group's lists need one array
     float clear_depth;
     uint32_t* out;         // width * height ARGB (device)
