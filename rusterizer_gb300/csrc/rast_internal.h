@@ -80,6 +80,9 @@ struct MeshRec {
     uint32_t* idx = nullptr;
     uint32_t nverts = 0, ntris = 0;
     bool live = false;
+    // a mesh that rast_mesh_update_async has updated: the end of the last frame that reads it, which
+    // the next update's copy waits for (frames of other meshes go on beside the copy)
+    cudaEvent_t used = nullptr;
     cudaEvent_t ready = nullptr;  // end of the last rast_mesh_update_async copy
     bool pending = false;         // that copy has not been waited for by a frame yet
     size_t bytes() const {
@@ -118,9 +121,10 @@ struct MeshRec {
         if (rgba) cudaFree(rgba);
         if (idx) cudaFree(idx);
         if (ready) cudaEventDestroy(ready);
+        if (used) cudaEventDestroy(used);
         pos = uv = rgba = nullptr;
         idx = nullptr;
-        ready = nullptr;
+        ready = used = nullptr;
         pending = false;
         live = false;
     }
@@ -293,8 +297,9 @@ struct rast_ctx {
     int tuned_tile[2] = {0, 0};             // batch autotuner: MSAA 1, MSAA 4
     std::vector<uint64_t> batch_hints;      // bins needed per scene by the last batch
     rast::DevBuf<uint32_t> batch_out;       // staging for host-pointer batch outputs
-    // asynchronous mesh updates: their copies run on `copy` after the frames enqueued before
-    // them (`frame_done`, recorded after every frame), and frames wait for the mesh's `ready`
+    // asynchronous mesh updates: their copies run on `copy` after the frames that read the mesh
+    // (MeshRec::used), and frames wait for the mesh's `ready`. `frame_done` is recorded after every
+    // frame once a readback needs it
     cudaStream_t copy = nullptr;
     cudaEvent_t frame_done = nullptr;
     bool frame_recorded = false;
