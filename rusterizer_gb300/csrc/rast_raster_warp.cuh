@@ -531,10 +531,14 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 :
     const uint32_t nsub = nsx * nsx;
     const uint32_t nlight = (sh.tq.busy - nheavy) * nsub;
     uint32_t shaded = 0, fsinv = 0, oobc = 0;
-    for (;;) {
-        uint32_t qi = 0;
-        if (lane == 0) qi = atomicAdd(&queue[2], 1u);
-        qi = __shfl_sync(0xFFFFFFFFu, qi, 0);
+    // with no more units than warps, one unit per warp by its place, SMs first (see k_raster)
+    const bool few = nlight <= gridDim.x * kWarpUnitWarps;
+    for (bool more = true; more; more = !few) {
+        uint32_t qi = warp * gridDim.x + blockIdx.x;
+        if (!few) {
+            if (lane == 0) qi = atomicAdd(&queue[2], 1u);
+            qi = __shfl_sync(0xFFFFFFFFu, qi, 0);
+        }
         if (qi >= nlight) break;
         const uint32_t gt = busy_tile(sh.tq, nheavy + qi / nsub), sub = qi % nsub;
         const FrameDev& f = frames[frame_of_tile(frames, nframes, gt)];
