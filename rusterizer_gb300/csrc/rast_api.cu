@@ -179,7 +179,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
             i = j;
         }
         // scratch
-        bool ok = E.vclip.reserve(small ? 0 : vtot) && E.vscr.reserve(vtot) && E.vcode.reserve(small ? 0 : vtot) &&
+        bool ok = E.vbin.reserve(small ? 0 : vtot) && E.vscr.reserve(vtot) &&
                   E.tri_rect.reserve(ttot) && E.tri_aux.reserve(ttot) &&
                   E.counts.reserve(count_tot) && E.tile_start.reserve(tile_tot) &&
                   E.tile_count.reserve(tile_tot) && E.tile_order.reserve((uint64_t)kOrderArrays * tile_tot) &&
@@ -233,9 +233,8 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         a.scan_groups = group_tot;
         a.max_tiles = max_tiles;
         Scratch& S = a.scratch;
-        S.vclip = E.vclip.p;
+        S.vbin = E.vbin.p;
         S.vscr = E.vscr.p;
-        S.vcode = E.vcode.p;
         S.tri_rect = E.tri_rect.p;
         S.tri_aux = E.tri_aux.p;
         S.counts = E.counts.p;

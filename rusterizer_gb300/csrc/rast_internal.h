@@ -191,8 +191,7 @@ struct DeviceState {
 
 struct Engine {
     cudaStream_t stream = nullptr;
-    DevBuf<float4> vclip, vscr;
-    DevBuf<uint16_t> vcode;
+    DevBuf<float4> vbin, vscr;
     DevBuf<unsigned long long> tri_rect;
     DevBuf<uint32_t> tri_aux, counts, tile_start, tile_count, tile_order, bins, qbins, qcount, clip_list;
     DevBuf<float> clip_store;

@@ -78,7 +78,7 @@ struct Carve {
 // Offsets of every buffer of one frame inside the scratch array, for the given bin and
 // clip-store capacities; `end` is the bytes used.
 struct Layout {
-    size_t state, frame, draw, chunks, vblocks, vclip, vscr, vcode, rect, aux, counts, tstart, tcount,
+    size_t state, frame, draw, chunks, vblocks, vbin, vscr, rect, aux, counts, tstart, tcount,
         torder, bins, qbins, qcount, clip, clist, end;
 };
 
@@ -93,9 +93,9 @@ Layout carve_layout(uint32_t nverts, uint32_t ntris, uint32_t nchunks, uint32_t 
     L.draw = c.take(sizeof(DrawDev));
     L.chunks = c.take(sizeof(ChunkDev) * (nchunks ? nchunks : 1));
     L.vblocks = c.take(sizeof(uint2) * (nvb ? nvb : 1));
-    L.vclip = c.take(sizeof(float4) * (size_t)nverts);
+    L.vbin = c.take(sizeof(float4) * (size_t)nverts);
     L.vscr = c.take(sizeof(float4) * (size_t)nverts);
-    L.vcode = c.take(sizeof(uint16_t) * (size_t)nverts);
+    c.take(sizeof(uint16_t) * (size_t)nverts);  // unused: the frames that fit the array stay the same
     L.rect = c.take(sizeof(unsigned long long) * (size_t)ntris);
     L.aux = c.take(sizeof(uint32_t) * (size_t)ntris);
     L.counts = c.take(sizeof(uint32_t) * (size_t)count_chunks * ntiles);
@@ -255,9 +255,8 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
         a.raster_queue = dstate->queue;
         a.raster_heavy_bits = kDefaultHeavyBits;
         Scratch& S = a.scratch;
-        S.vclip = reinterpret_cast<float4*>(base + L.vclip);
+        S.vbin = reinterpret_cast<float4*>(base + L.vbin);
         S.vscr = reinterpret_cast<float4*>(base + L.vscr);
-        S.vcode = reinterpret_cast<uint16_t*>(base + L.vcode);
         S.tri_rect = reinterpret_cast<unsigned long long*>(base + L.rect);
         S.tri_aux = reinterpret_cast<uint32_t*>(base + L.aux);
         S.counts = reinterpret_cast<uint32_t*>(base + L.counts);

@@ -4,9 +4,9 @@
 // draws. Plain rendering is one frame; the batched and serving paths pass many.
 //
 // HBM layout (all scratch owned by the context, grown on demand, never per frame):
-//   vclip[v]  float4  clip-space position of vertex v (MVP * (x,y,z,1))
+//   vbin[v]   float4  what binning reads of vertex v: clip x, y and screen x, y, or the clip predicates
+//                     in place of clip x (rast_kernels.cu vertex_bin)
 //   vscr[v]   float4  (screen x, screen y, screen z, w) after divide + viewport
-//   vcode[v]  u16     clip predicates (rast_device.cuh clip_code)
 //   tri_rect[t] u64   pixel box of triangle t (x0,y0,x1,y1 inclusive, 16 bits each),
 //                     kRectEmpty when culled; bit 63: clipped
 //   tri_aux[t]  u32   offset of the clipped polygon in clip_store, kNone when unclipped
@@ -160,9 +160,8 @@ struct ChunkDev {
 };
 
 struct Scratch {
-    float4* vclip;
+    float4* vbin;
     float4* vscr;
-    uint16_t* vcode;
     unsigned long long* tri_rect;
     uint32_t* tri_aux;
     uint32_t* counts;
