@@ -1122,7 +1122,9 @@ struct alignas(16) RasterSmem {
     // item | pixel << 8 | depth mask << 16, and sample 0's depth
     uint32_t sq[kRasterWarps][C::QC];
     float sz0[kRasterWarps][C::QC];
-    int rowd[TS + 1], cold[TS + 1];  // candidate work of the batch, difference arrays
+    // candidate work of the batch by row (low half) and by column (high half), as differences; the
+    // sums stay below 2^16 (at most 128 items of 16 pixels)
+    uint32_t work[TS + 1];
     uint32_t tmp[40];
     uint32_t misc[8];  // [0] unit ticket, [1] items staged, [2..4] statistics, [5] the unit's bin
     TileQueue tq;
@@ -1310,11 +1312,11 @@ __device__ __forceinline__ void stage_entry(RasterSmem<S, TS>& sm, const FrameDe
         if (nonempty) {
             const uint32_t lx0 = cx0 - X0, ly0 = cy0 - Y0, lx1 = cx1 - X0, ly1 = cy1 - Y0;
             r = lx0 | (ly0 << 8) | (lx1 << 16) | (ly1 << 24);
-            const int cw = (int)(lx1 - lx0), chh = (int)(ly1 - ly0);
-            atomicAdd(&sm.rowd[ly0], cw);
-            atomicAdd(&sm.rowd[ly1], -cw);
-            atomicAdd(&sm.cold[lx0], chh);
-            atomicAdd(&sm.cold[lx1], -chh);
+            const uint32_t cw = lx1 - lx0, ch = (ly1 - ly0) << 16;
+            atomicAdd(&sm.work[ly0], cw);
+            atomicAdd(&sm.work[ly1], 0u - cw);
+            atomicAdd(&sm.work[lx0], ch);
+            atomicAdd(&sm.work[lx1], 0u - ch);
         }
         sm.irect[it] = r;
         sm.itri[it] = g;
@@ -1329,26 +1331,20 @@ __device__ __forceinline__ void stage_entry(RasterSmem<S, TS>& sm, const FrameDe
 // item meets each warp on at most TS / kRasterWarps lines. Returns 0 for rows, 1 for columns.
 // Called by one warp.
 template <int TS>
-__device__ __forceinline__ uint32_t split_work(const int* rowd, const int* cold) {
+__device__ __forceinline__ uint32_t split_work(const uint32_t* work) {
     const uint32_t lane = lane_id();
-    // per-line work from the difference arrays (lane = line)
-    int rw = lane < (uint32_t)TS ? rowd[lane] : 0, cw = lane < (uint32_t)TS ? cold[lane] : 0;
+    // per-line work from the differences (lane = line), rows and columns in one word
+    uint32_t w = lane < (uint32_t)TS ? work[lane] : 0u;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xFFFFFFFFu, rw, o), z = __shfl_up_sync(0xFFFFFFFFu, cw, o);
-        if (lane >= (uint32_t)o) {
-            rw += y;
-            cw += z;
-        }
+    for (int o = 1; o < TS; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
+        if (lane >= (uint32_t)o) w += y;
     }
-    uint32_t wr = lane < (uint32_t)TS ? (uint32_t)rw : 0u;
-    uint32_t wc = lane < (uint32_t)TS ? (uint32_t)cw : 0u;
+    if (lane >= (uint32_t)TS) w = 0;
     // each warp's load: the sum of its lines (lane % kRasterWarps), then the heaviest warp
 #pragma unroll
-    for (int o = kRasterWarps; o < 32; o <<= 1) {
-        wr += __shfl_down_sync(0xFFFFFFFFu, wr, o);
-        wc += __shfl_down_sync(0xFFFFFFFFu, wc, o);
-    }
+    for (int o = kRasterWarps; o < TS; o <<= 1) w += __shfl_down_sync(0xFFFFFFFFu, w, o);
+    uint32_t wr = w & 0xFFFFu, wc = w >> 16;
 #pragma unroll
     for (int o = kRasterWarps / 2; o > 0; o >>= 1) {
         wr = max(wr, __shfl_xor_sync(0xFFFFFFFFu, wr, o));
@@ -1645,8 +1641,7 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
     while (pos < nent) {
         // ---- A. fill a batch with the items of the next entries that touch this tile
         if (threadIdx.x <= (uint32_t)TS) {
-            sm.rowd[threadIdx.x] = 0;
-            sm.cold[threadIdx.x] = 0;
+            sm.work[threadIdx.x] = 0;
         }
         // largest depth stored in the tile before this batch, for depth_cull: the clear depth
         // for the unit's first batch; else reduced here and combined after the scan's barriers.
@@ -1703,23 +1698,38 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
         // choice from the batch's work histograms: no barrier to wait for one warp's), and list
         // this warp's spans in submission order: its lines of each item's box (rows, or columns
         // in column mode: line l belongs to warp l % kRasterWarps)
-        const uint32_t mode = __shfl_sync(0xFFFFFFFFu, split_work<TS>(sm.rowd, sm.cold), 0);
+        const uint32_t mode = __shfl_sync(0xFFFFFFFFu, split_work<TS>(sm.work), 0);
         uint32_t nspan = 0;
+        const uint32_t lsh = mode ? 0u : 8u;
         for (uint32_t i0 = 0; i0 < nit; i0 += 32) {
             const uint32_t it = i0 + lane;
-            uint32_t first = 0, nl = 0;
-            if (it < nit) {
-                const uint32_t r = sm.irect[it];
-                const uint32_t l0 = (mode ? r : r >> 8) & 0xFFu, l1 = (mode ? r >> 16 : r >> 24) & 0xFFu;
-                first = l0 + ((warp - l0) & (kRasterWarps - 1));
-                nl = first < l1 ? (l1 - first + kRasterWarps - 1) / kRasterWarps : 0u;
+            const uint32_t r = it < nit ? sm.irect[it] : 0u;
+            const uint32_t l0 = (r >> lsh) & 0xFFu, l1 = (r >> (lsh + 16)) & 0xFFu;
+            // the warp's first line at or past l0, and how many it has before l1 (0 for an empty box)
+            const uint32_t first = l0 + ((warp - l0) & (kRasterWarps - 1));
+            const uint32_t nl = (l1 + (uint32_t)kRasterWarps - 1 - first) / kRasterWarps;
+            const uint32_t lt = lanemask_lt();
+            const uint32_t n1 = __ballot_sync(0xFFFFFFFFu, nl & 1u);
+            uint32_t at = nspan + __popc(n1 & lt);
+            nspan += __popc(n1);
+            if (C::LINES > 1) {
+                const uint32_t n2 = __ballot_sync(0xFFFFFFFFu, nl & 2u);
+                if (n2) {
+                    at += 2 * __popc(n2 & lt);
+                    nspan += 2 * __popc(n2);
+                }
             }
-            const uint32_t n1 = __ballot_sync(0xFFFFFFFFu, nl & 1u), n2 = __ballot_sync(0xFFFFFFFFu, nl & 2u),
-                           n4 = __ballot_sync(0xFFFFFFFFu, nl & 4u), lt = lanemask_lt();
-            const uint32_t at = nspan + __popc(n1 & lt) + 2 * __popc(n2 & lt) + 4 * __popc(n4 & lt);
-            for (uint32_t k = 0; k < nl; ++k)
-                sm.span[warp][at + k] = (uint16_t)(it | ((first + k * kRasterWarps) << 8));
-            nspan += __popc(n1) + 2 * __popc(n2) + 4 * __popc(n4);
+            if (C::LINES > 3) {
+                const uint32_t n4 = __ballot_sync(0xFFFFFFFFu, nl & 4u);
+                if (n4) {
+                    at += 4 * __popc(n4 & lt);
+                    nspan += 4 * __popc(n4);
+                }
+            }
+            const uint32_t e = it | (first << 8);
+#pragma unroll
+            for (uint32_t k = 0; k < (uint32_t)C::LINES; ++k)
+                if (k < nl) sm.span[warp][at + k] = (uint16_t)(e + ((k * kRasterWarps) << 8));
         }
         __syncwarp();
         // ---- C. per warp, in submission order: its spans 32 at a time, one per lane, each
