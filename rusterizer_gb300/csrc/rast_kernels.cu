@@ -1077,6 +1077,14 @@ __device__ __forceinline__ uint32_t heavy_tiles(const TileQueue& tq, uint32_t he
     return h >= (uint32_t)kClasses ? 0u : tq.end[kClasses - 1 - h];
 }
 
+// Strips of rows that each raster unit is divided into, a CTA (or warp) each, when there are fewer units
+// than places for them: every strip stages all of the unit's entries, so this pays only where the GPU
+// would wait for a few units' serial batches.
+// Returns log2 of their number. A 256-triangle sphere at 256x192: 57 -> 50 us a frame.
+__device__ __forceinline__ uint32_t strips_for(uint32_t nunits, uint32_t places) {
+    return 4 * nunits <= places ? 2u : 2 * nunits <= places ? 1u : 0u;
+}
+
 // A raster CTA owns one TS x TS tile: a whole bin (bin edge == TS) or one quadrant of a bin
 // twice as wide. Bin entries carry, in their low 4 bits, the quadrants the triangle's pixel box
 // touches, so a quadrant CTA skips the other entries without loading them.
@@ -1126,7 +1134,7 @@ struct alignas(16) RasterSmem {
     // sums stay below 2^16 (at most 128 items of 16 pixels)
     uint32_t work[TS + 1];
     uint32_t tmp[40];
-    uint32_t misc[8];  // [0] unit ticket, [1] items staged, [2..4] statistics, [5] the unit's bin
+    uint32_t misc[8];  // [0] unit ticket, [1] items staged, [2..4] statistics, [5] the unit's bin, [6] log2 of the strips
     TileQueue tq;
     uint32_t zmaxw[kRasterWarps];  // per warp: largest stored depth of its share of the tile
 };
@@ -1263,7 +1271,7 @@ template <int S, int TS>
 __device__ __forceinline__ void stage_entry(RasterSmem<S, TS>& sm, const FrameDev& f,
                                             const DrawDev* __restrict__ draws, const Scratch& s,
                                             uint32_t g, uint32_t aux, uint32_t nitems, uint32_t first,
-                                            uint32_t X0, uint32_t Y0, float ztile) {
+                                            uint32_t X0, uint32_t Y0, uint32_t row0, uint32_t row1, float ztile) {
     const uint32_t di = find_draw(draws, f, g);
     const DrawDev& d = draws[di];
     const int fs = d.fs;
@@ -1303,7 +1311,7 @@ __device__ __forceinline__ void stage_entry(RasterSmem<S, TS>& sm, const FrameDe
         uint32_t bx0, bx1, by0, by1;
         pixel_bbox(sv, f.width, f.height, bx0, bx1, by0, by1);
         const uint32_t cx0 = max(bx0, X0), cx1 = min(bx1, X0 + TS);
-        const uint32_t cy0 = max(by0, Y0), cy1 = min(by1, Y0 + TS);
+        const uint32_t cy0 = max(by0, Y0 + row0), cy1 = min(by1, Y0 + row1);
         // hidden: no sample depth can get below the largest depth stored in the tile
         // (depth_cull), so the strict depth test (mod.rs:363-378) fails everywhere
         const bool nonempty = bx0 < bx1 && by0 < by1 && cx0 < cx1 && cy0 < cy1 &&
@@ -1600,18 +1608,22 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
     // i takes unit i and no other: from the counter, the CTAs of the SMs nearest to it take up to
     // seven before the far ones get any (2 000-triangle soup 86 -> 80 us a frame). With more units the
     // counter is the better one (a CTA that starts late would hold a heavy unit: 100k soup 290 -> 319).
-    const uint32_t nunits = heavy_tiles(sm.tq, frames[0].heavy_bits) * nsub;
+    const uint32_t nwhole = heavy_tiles(sm.tq, frames[0].heavy_bits) * nsub;
+    const uint32_t nunits = nwhole << strips_for(nwhole, gridDim.x);
+    if (threadIdx.x == 0) sm.misc[6] = strips_for(nwhole, gridDim.x);
     if (threadIdx.x == 0) {
         const uint32_t qi = nunits <= gridDim.x ? blockIdx.x : atomicAdd(&queue[0], 1u);
         sm.misc[0] = qi;
-        if (qi < nunits) sm.misc[5] = busy_tile(sm.tq, qi / nsub);
+        if (qi < nunits) sm.misc[5] = busy_tile(sm.tq, (qi >> sm.misc[6]) / nsub);
     }
     for (;;) {
     __syncthreads();
     // misc[0] and misc[5] are written again only after this unit's resolve, many barriers later
     const uint32_t qi = sm.misc[0];
     if (qi >= nunits) break;
-    const uint32_t gt = sm.misc[5], sub = qi % nsub;
+    const uint32_t gt = sm.misc[5], ssh = sm.misc[6], sub = (qi >> ssh) % nsub;
+    // the unit's rows of the tile, first | end << 8 (one register through the candidate loop)
+    const uint32_t rows = (qi & ((1u << ssh) - 1u)) * (TS >> ssh) * 0x101u + ((TS >> ssh) << 8);
     const FrameDev& f = frames[frame_of_tile(frames, nframes, gt)];
     const uint32_t lt = gt - f.tile_begin;
     const uint32_t X0 = (lt % f.tiles_x) * (uint32_t)f.ts + (sub % nsx) * TS;
@@ -1620,10 +1632,11 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
     {
         const float4 zc = make_float4(f.clear_depth, f.clear_depth, f.clear_depth, f.clear_depth);
         const uint4 cc = make_uint4(kClearColor, kClearColor, kClearColor, kClearColor);
-        for (uint32_t i = threadIdx.x; i < (uint32_t)(C::NPIX * S / 4); i += blockDim.x) {
+        // the colours of other rows are not read, nor their depths
+        for (uint32_t i = (rows & 0xFFu) * (TS * S / 4) + threadIdx.x; i < (rows >> 8) * (TS * S / 4); i += blockDim.x)
             reinterpret_cast<float4*>(sm.zb)[i] = zc;
+        for (uint32_t i = threadIdx.x; i < (uint32_t)(C::NPIX * S / 4); i += blockDim.x)
             reinterpret_cast<uint4*>(sm.cb)[i] = cc;
-        }
     }
     // the bin's entries, or for a quadrant of a 32-pixel bin its own split list
     uint32_t nent;
@@ -1650,7 +1663,7 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
         bool zt_ready = s.log || pos == 0;
         if (!zt_ready) {
             uint32_t zm = 0;
-            for (uint32_t i = threadIdx.x; i < (uint32_t)(C::NPIX * S); i += blockDim.x)
+            for (uint32_t i = (rows & 0xFFu) * (TS * S) + threadIdx.x; i < (rows >> 8) * (TS * S); i += blockDim.x)
                 zm = max(zm, float_to_ordered(sm.zb[i]));
             zm = __reduce_max_sync(0xFFFFFFFFu, zm);
             if (lane == 0) sm.zmaxw[warp] = zm;
@@ -1686,7 +1699,7 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
                     zt = ordered_to_float(zm);
                     zt_ready = true;
                 }
-                stage_entry<S, TS>(sm, f, draws, s, g, aux, nitems, nit + iex, X0, Y0, zt);
+                stage_entry<S, TS>(sm, f, draws, s, g, aux, nitems, nit + iex, X0, Y0, rows & 0xFFu, rows >> 8, zt);
             }
             __syncthreads();
             nit = sm.misc[1];
@@ -1819,7 +1832,7 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
     __syncthreads();
     uint32_t next_ticket = nunits;
     if (threadIdx.x == 0 && nunits > gridDim.x) next_ticket = atomicAdd(&queue[0], 1u);
-    for (uint32_t p = threadIdx.x; p < (uint32_t)C::NPIX; p += blockDim.x) {
+    for (uint32_t p = (rows & 0xFFu) * TS + threadIdx.x; p < (rows >> 8) * TS; p += blockDim.x) {
         const uint32_t x = X0 + p % TS, y = Y0 + p / TS;
         if (x >= W || y >= H) continue;
         const unsigned long long o = (unsigned long long)y * W + x;
@@ -1837,7 +1850,7 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
     }
     if (threadIdx.x == 0) {
         sm.misc[0] = next_ticket;
-        if (next_ticket < nunits) sm.misc[5] = busy_tile(sm.tq, next_ticket / nsub);
+        if (next_ticket < nunits) sm.misc[5] = busy_tile(sm.tq, (next_ticket >> sm.misc[6]) / nsub);
     }
     }  // units with entries
 
@@ -2059,7 +2072,8 @@ static cudaError_t launch_raster_t(const LaunchArgs& a, uint32_t nsx) {
     }
     if (a.raster_blocks == 0) return cudaSuccess;
     const uint32_t* order = a.scratch.tile_order + (unsigned long long)kOrderArrays * a.raster_tile_offset;
-    const unsigned long long units = (unsigned long long)a.raster_blocks * nsx * nsx;
+    // as many CTAs as there could be strips of units
+    const unsigned long long units = 4ull * a.raster_blocks * nsx * nsx;
     // heavy tiles CTA-wide (none when every bin is below the threshold: the launch then only
     // helps with the bins without entries), then the light tiles one warp each
     if (a.raster_heavy_bits < 32) {

@@ -14,24 +14,22 @@
 
 constexpr int kWarpUnitWarps = 4;  // warps (independent tiles) per CTA of k_raster_warp
 // CTAs per SM the launch bounds aim at: with 4 samples the shared sample tiles allow 5; with
-// one sample 6 (79 registers, no spills; 7 spills and ran 2% slower on the scene mix, 5 3% slower)
+// one sample registers do (6 would spill)
 constexpr int kWarpUnitCtas = 5;
-constexpr int kWarpUnitCtas1 = 6;
+constexpr int kWarpUnitCtas1 = 5;
 
 template <int S, int TS>
 struct alignas(16) WarpUnitSmem {
     static constexpr int NPIX = TS * TS;
     static constexpr int IB = 32;  // items per batch (one per lane)
     static constexpr int QC = 64;  // ring entries
-    float zb[NPIX * S];            // sample-major: sample k of pixel p at k * NPIX + p
-    uint32_t cb[NPIX * S];
-    uint8_t rpre[IB][TS];          // rows trimmed by line_span: candidates before each box row
-                                   // (at most 15 rows of 16 before the last: fits a byte)
-    uint8_t rsta[IB][TS];          // rows trimmed by line_span: first column of each box row
-    float qz[S][QC];               // ring of covered fragments, in submission order
-    uint8_t qitem[QC], qpix[QC], qcov[QC];
-    float sz0[QC];                 // ring of depth-passed fragments waiting for the shader
-    uint8_t sitem[QC], spix[QC], sdm[QC];
+    float zb[NPIX * S];            // pixel-major: the samples of pixel p at p * S
+    uint32_t cb[NPIX * S];         // sample-major: sample k of pixel p at k * NPIX + p
+    float qz[QC][S];               // sample depths of the fragment ring, NaN where not covered
+    uint2 run[32];                 // non-empty spans of a group: start, item | row << 8 | first column << 16
+    uint32_t q[QC];   // ring of covered fragments, in submission order: item | pixel << 8 | mask << 16
+    uint32_t sq[QC];  // ring of depth-passed fragments waiting for the shader: item | pixel << 8 | mask << 16
+    uint8_t rowed[IB];  // items with rows, in order
 };
 
 template <int S, int TS>
@@ -67,7 +65,7 @@ struct WItem {
 template <int TS>
 __device__ __forceinline__ void wstage_item(WItem& it, const FrameDev& f, const DrawDev* __restrict__ draws,
                                             const Scratch& s, uint32_t g, uint32_t aux, uint32_t k, uint32_t X0,
-                                            uint32_t Y0, float ztile) {
+                                            uint32_t Y0, uint32_t row0, uint32_t row1, float ztile) {
     const uint32_t di = find_draw(draws, f, g);
     const DrawDev& d = draws[di];
     float4 sv[3];
@@ -110,7 +108,7 @@ __device__ __forceinline__ void wstage_item(WItem& it, const FrameDev& f, const 
     uint32_t bx0, bx1, by0, by1;
     pixel_bbox(sv, f.width, f.height, bx0, bx1, by0, by1);
     const uint32_t cx0 = max(bx0, X0), cx1 = min(bx1, X0 + TS);
-    const uint32_t cy0 = max(by0, Y0), cy1 = min(by1, Y0 + TS);
+    const uint32_t cy0 = max(by0, Y0 + row0), cy1 = min(by1, Y0 + row1);
     // hidden items (depth_cull) cover nothing that could pass the strict depth test
     const bool nonempty = bx0 < bx1 && by0 < by1 && cx0 < cx1 && cy0 < cy1 &&
                           !depth_cull(sv[0].z, sv[1].z, sv[2].z, ztile);
@@ -132,48 +130,46 @@ __device__ __forceinline__ void wdepth(WarpUnitSmem<S, TS>& sm, const WItem& my,
     const uint32_t lane = lane_id();
     const bool valid = lane < n;
     const uint32_t q = (head + lane) & (U::QC - 1);
-    uint32_t it = 0, pix = 0, cov = 0;
+    uint32_t fr = 0;
     float z[S];
 #pragma unroll
     for (int k = 0; k < S; ++k) z[k] = 0.0f;
     if (valid) {
-        it = sm.qitem[q];
-        pix = sm.qpix[q];
-        cov = sm.qcov[q];
-#pragma unroll
-        for (int k = 0; k < S; ++k) z[k] = sm.qz[k][q];
+        fr = sm.q[q];
+        load_samples<S>(sm.qz[q], z);
     }
     // the fragment log (debug) names the fragment's triangle: read from the item's lane
     uint32_t ltri = 0, lmeta = 0;
     if (s.log) {
-        ltri = shfl_u(my.tri, it);
-        lmeta = shfl_u(my.meta, it);
+        ltri = shfl_u(my.tri, fr & 31u);
+        lmeta = shfl_u(my.meta, fr & 31u);
     }
+    const uint32_t pix = (fr >> 8) & 0xFFu;
     const uint32_t key = valid ? pix : 0x10000u + lane;
     const uint32_t grp = __match_any_sync(0xFFFFFFFFu, key);
     const uint32_t rank = __popc(grp & lanemask_lt());
     const uint32_t maxr = __reduce_max_sync(0xFFFFFFFFu, rank);
     uint32_t dm = 0;
     for (uint32_t r = 0; r <= maxr; ++r) {
-        const bool act = valid && rank == r;
+        if (valid && rank == r) {
+            float old[S];
+            load_samples<S>(&sm.zb[pix * S], old);
 #pragma unroll
-        for (int k = 0; k < S; ++k) {
-            const float old = sm.zb[k * U::NPIX + pix];
-            const bool pass = act & (((cov >> k) & 1u) != 0) & (z[k] < old);
-            if (pass) sm.zb[k * U::NPIX + pix] = z[k];
-            dm |= (uint32_t)pass << k;
+            for (int k = 0; k < S; ++k) {
+                const bool pass = z[k] < old[k];
+                old[k] = pass ? z[k] : old[k];
+                dm |= pass ? 1u << k : 0u;
+            }
+            store_samples<S>(&sm.zb[pix * S], old);
+            if (s.log)
+                log_fragment(s, ltri, lmeta & 0xFFu, ((Y0 + pix / TS) << 16) | (X0 + pix % TS),
+                             (dm << 8) | (fr >> 16));
         }
-        if (s.log && act)
-            log_fragment(s, ltri, lmeta & 0xFFu, ((Y0 + pix / TS) << 16) | (X0 + pix % TS), (dm << 8) | cov);
         __syncwarp();
     }
     const uint32_t bal = __ballot_sync(0xFFFFFFFFu, dm != 0);
     if (dm) {
-        const uint32_t sq = (stail + __popc(bal & lanemask_lt())) & (U::QC - 1);
-        sm.sitem[sq] = (uint8_t)it;
-        sm.spix[sq] = (uint8_t)pix;
-        sm.sdm[sq] = (uint8_t)dm;
-        sm.sz0[sq] = (cov & 1u) ? z[0] : 0.0f;
+        sm.sq[(stail + __popc(bal & lanemask_lt())) & (U::QC - 1)] = (fr & 0xFFFFu) | (dm << 16);
         shaded += __popc(dm);
         fsinv += 1;
     }
@@ -190,8 +186,8 @@ __device__ __forceinline__ void wshade(WarpUnitSmem<S, TS>& sm, const WItem& my,
     using U = WarpUnitSmem<S, TS>;
     const uint32_t lane = lane_id();
     const bool valid = lane < n;
-    const uint32_t q = (head + lane) & (U::QC - 1);
-    const uint32_t it = valid ? sm.sitem[q] : 0u;
+    const uint32_t fr = valid ? sm.sq[(head + lane) & (U::QC - 1)] : 0u;
+    const uint32_t it = fr & 31u;
     float px[3], py[3], w[3], tuv[6];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -202,10 +198,16 @@ __device__ __forceinline__ void wshade(WarpUnitSmem<S, TS>& sm, const WItem& my,
 #pragma unroll
     for (int k = 0; k < 6; ++k) tuv[k] = shfl_f(my.uv[k], it);
     const uint32_t meta = shfl_u(my.meta, it), tri = shfl_u(my.tri, it);
-    uint32_t argb = 0, pix = 0, dm = 0;
+    const uint32_t pix = (fr >> 8) & 0xFFu, dm = fr >> 16;
+    // FS::Debug reads sample 0's depth, computed again
+    float z[3] = {0.0f, 0.0f, 0.0f}, inv = 0.0f;
+    if (__any_sync(0xFFFFFFFFu, valid && draws[meta >> 8].fs == 2)) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) z[k] = shfl_f(my.z[k], it);
+        inv = shfl_f(my.inv, it);
+    }
+    uint32_t argb = 0;
     if (valid) {
-        pix = sm.spix[q];
-        dm = sm.sdm[q];
         float xs, ys;
         interp_point<S>(X0 + pix % TS, Y0 + pix / TS, dm, xs, ys);
         float u, v, ww;
@@ -225,8 +227,11 @@ __device__ __forceinline__ void wshade(WarpUnitSmem<S, TS>& sm, const WItem& my,
 #pragma unroll
                 for (int c = 0; c < 4; ++c) col[c] = vc[0][c] * u + vc[1][c] * v + vc[2][c] * ww;
             } else {
-                // FS::Debug (upstream src/main.rs:218-220): grayscale(frag_coords.depths[0])
-                const float z0 = sm.sz0[q];
+                // FS::Debug (upstream src/main.rs:218-220): grayscale(frag_coords.depths[0]), 0 where
+                // sample 0 is not covered
+                const Cover<S> cv = cover_pixel<S>(px[0], py[0], px[1], py[1], px[2], py[2], inv, z[0], z[1], z[2],
+                                                   (float)(X0 + pix % TS), (float)(Y0 + pix / TS));
+                const float z0 = (cv.mask & 1u) ? cv.z[0] : 0.0f;
                 col[0] = z0;
                 col[1] = z0;
                 col[2] = z0;
@@ -252,14 +257,15 @@ __device__ __forceinline__ void wshade(WarpUnitSmem<S, TS>& sm, const WItem& my,
 // warp's tile: four consecutive pixels of a row per lane with 16-byte stores where the image
 // row allows them, one pixel per lane otherwise (image edges, unaligned outputs, sample capture).
 template <int S, int TS>
-__device__ __forceinline__ void wresolve(const WarpUnitSmem<S, TS>& sm, const FrameDev& f, uint32_t X0, uint32_t Y0) {
+__device__ __forceinline__ void wresolve(const WarpUnitSmem<S, TS>& sm, const FrameDev& f, uint32_t X0, uint32_t Y0,
+                                         uint32_t row0, uint32_t row1) {
     using U = WarpUnitSmem<S, TS>;
     const uint32_t lane = lane_id();
     const uint32_t W = f.width, H = f.height;
     const bool vec = !f.dbg_depth && (W & 3u) == 0 && X0 + TS <= W &&
                      (reinterpret_cast<uintptr_t>(f.out) & 15u) == 0;
     if (vec) {
-        for (uint32_t p = 4 * lane; p < (uint32_t)U::NPIX; p += 128) {
+        for (uint32_t p = row0 * TS + 4 * lane; p < row1 * TS; p += 128) {
             const uint32_t y = Y0 + p / TS;
             if (y >= H) break;  // rows go down with p
             uint4 c[S];
@@ -278,7 +284,7 @@ __device__ __forceinline__ void wresolve(const WarpUnitSmem<S, TS>& sm, const Fr
         }
         return;
     }
-    for (uint32_t p = lane; p < (uint32_t)U::NPIX; p += 32) {
+    for (uint32_t p = row0 * TS + lane; p < row1 * TS; p += 32) {
         const uint32_t x = X0 + p % TS, y = Y0 + p / TS;
         if (x >= W || y >= H) continue;
         const unsigned long long o = (unsigned long long)y * W + x;
@@ -289,7 +295,7 @@ __device__ __forceinline__ void wresolve(const WarpUnitSmem<S, TS>& sm, const Fr
         if (f.dbg_depth) {
 #pragma unroll
             for (int k = 0; k < S; ++k) {
-                f.dbg_depth[o * S + k] = sm.zb[k * U::NPIX + p];
+                f.dbg_depth[o * S + k] = sm.zb[p * S + k];
                 f.dbg_color[o * S + k] = sm.cb[k * U::NPIX + p];
             }
         }
@@ -308,8 +314,8 @@ template <int S, int TS>
 __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const FrameDev& f,
                                           const DrawDev* __restrict__ draws, const Scratch& s,
                                           const uint32_t* __restrict__ bins, uint32_t nent, uint32_t mybit,
-                                          uint32_t X0, uint32_t Y0, uint32_t& shaded, uint32_t& fsinv,
-                                          uint32_t& oobc) {
+                                          uint32_t X0, uint32_t Y0, uint32_t row0, uint32_t row1,
+                                          uint32_t& shaded, uint32_t& fsinv, uint32_t& oobc) {
     using U = WarpUnitSmem<S, TS>;
     const uint32_t lane = lane_id();
     {
@@ -332,7 +338,8 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const FrameDe
         // the largest stored depth, refreshed before batches 1, 2, 4, 8, ...
         if (!s.log && batch > 0 && (batch & (batch - 1)) == 0) {
             uint32_t zm = 0;
-            for (uint32_t i = lane; i < (uint32_t)(U::NPIX * S); i += 32) zm = max(zm, float_to_ordered(sm.zb[i]));
+            for (uint32_t i = row0 * (TS * S) + lane; i < row1 * (TS * S); i += 32)
+                zm = max(zm, float_to_ordered(sm.zb[i]));
             zt = ordered_to_float(__reduce_max_sync(0xFFFFFFFFu, zm));
         }
         ++batch;
@@ -371,130 +378,97 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const FrameDe
             src = min(src, 31u);
             const uint32_t sg = __shfl_sync(0xFFFFFFFFu, g, src), saux = __shfl_sync(0xFFFFFFFFu, aux, src);
             const uint32_t sk = qi - (__shfl_sync(0xFFFFFFFFu, incl, src) - __shfl_sync(0xFFFFFFFFu, nitems, src));
-            if (lane >= nit && lane < nit + win) wstage_item<TS>(my, f, draws, s, sg, saux, sk, X0, Y0, zt);
+            if (lane >= nit && lane < nit + win) wstage_item<TS>(my, f, draws, s, sg, saux, sk, X0, Y0, row0, row1, zt);
             nit += win;
             pos += take;
             if (take < 32) break;  // the batch is full, or the entries ran out
         }
-        // ---- B. candidates of each item (lane = item): the whole box, or for boxes of kTrimMin+
-        // columns each row trimmed by line_span
-        uint32_t c = 0, geo = 0, nrows = 0;  // geo: x0 | y0 << 5 | w << 10 | h << 16 | trimmed << 21
+        // ---- B. the rows of the items' boxes in submission order, 32 at a time, one span per lane (a
+        // lane finds its item by counting the marks of the items that start up to its row): boxes of
+        // kTrimMin+ columns trimmed by line_span_pts; the non-empty spans go to `run`
+        uint32_t geo = 0, nrows = 0;  // x0 | y0 << 8 | x1 << 16
         if (lane < nit) {
-            const uint32_t r = my.rect;
-            const uint32_t x0 = r & 0xFFu, y0 = (r >> 8) & 0xFFu, x1 = (r >> 16) & 0xFFu, y1 = r >> 24;
-            const uint32_t w = x1 - x0, h = y1 - y0;
-            const bool trim = w >= kTrimMin && h > 0;
-            nrows = trim ? h : 0u;
-            c = w * h;
-            geo = x0 | (y0 << 5) | (w << 10) | (h << 16) | ((uint32_t)trim << 21);
+            geo = my.rect & 0xFFFFFFu;
+            nrows = (my.rect >> 24) - ((my.rect >> 8) & 0xFFu);
         }
-        // the rows to trim, spread over the lanes 32 at a time (a warp would otherwise run as many
-        // rounds as its tallest item has rows): task t is row t - (rows of earlier items) of the
-        // item whose running row count first exceeds t, read from that item's lane; the span's
-        // start goes to rsta, its length to rpre until the prefix pass below
         const uint32_t rincl = warp_incl_scan(nrows);
         const uint32_t rtot = __shfl_sync(0xFFFFFFFFu, rincl, 31);
-        for (uint32_t tb = 0; tb < rtot; tb += 32) {
-            const uint32_t t = tb + lane;
-            uint32_t j = 0;
-#pragma unroll
-            for (int st = 16; st > 0; st >>= 1) {
-                const uint32_t v = __shfl_sync(0xFFFFFFFFu, rincl, j + st - 1);
-                if (v <= t) j += st;
-            }
-            j = min(j, 31u);
-            const float px[3] = {shfl_f(my.px[0], j), shfl_f(my.px[1], j), shfl_f(my.px[2], j)};
-            const float py[3] = {shfl_f(my.py[0], j), shfl_f(my.py[1], j), shfl_f(my.py[2], j)};
-            const bool finite = fabsf(shfl_f(my.inv, j)) <= FLT_MAX;
-            const uint32_t gj = __shfl_sync(0xFFFFFFFFu, geo, j);
-            const uint32_t row = t - __shfl_sync(0xFFFFFFFFu, rincl - nrows, j);
-            if (t < rtot) {
-                const uint32_t x0 = gj & 31u, y0 = (gj >> 5) & 31u;
-                uint32_t a0 = x0, a1 = x0 + ((gj >> 10) & 31u);
-                if (finite) line_span_pts<S, TS>(px, py, 0u, y0 + row, X0, Y0, a0, a1);
-                sm.rsta[j][row] = (uint8_t)a0;
-                sm.rpre[j][row] = (uint8_t)(a1 - a0);
-            }
-        }
+        const uint32_t rowed = __ballot_sync(0xFFFFFFFFu, nrows != 0);
+        const uint32_t rstart = nrows ? rincl - nrows : 0xFFFFFFFFu;
+        if (nrows) sm.rowed[__popc(rowed & lanemask_lt())] = (uint8_t)lane;
         __syncwarp();
-        if (nrows) {
-            uint32_t run = 0;  // candidates before each row
-            for (uint32_t row = 0; row < nrows; ++row) {
-                const uint32_t len = sm.rpre[lane][row];
-                sm.rpre[lane][row] = (uint8_t)run;
-                run += len;
-            }
-            c = run;
-        }
-        const uint32_t incl = warp_incl_scan(c);
-        const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-        __syncwarp();
-        // ---- C. the candidates, 32 at a time, in submission order
+        const uint32_t upto = lanemask_lt() | (1u << lane);
+        uint32_t rbefore = 0xFFFFFFFFu;  // items that start in earlier groups, less one
         uint32_t head = 0, tail = 0, shead = 0, stail = 0;
-        for (uint32_t pb = 0; pb < total; pb += 32) {
-            const uint32_t p = pb + lane;
-            uint32_t j = 0;  // source item: number of items whose inclusive count is <= p
-#pragma unroll
-            for (int st = 16; st > 0; st >>= 1) {
-                const uint32_t v = __shfl_sync(0xFFFFFFFFu, incl, j + st - 1);
-                if (v <= p) j += st;
-            }
-            const uint32_t it = min(j, 31u);
-            const uint32_t exc = __shfl_sync(0xFFFFFFFFu, incl - c, it);
-            const uint32_t gg = __shfl_sync(0xFFFFFFFFu, geo, it);
-            // the item's points, depths and 1 / 2x area from its lane
-            const float p0x = shfl_f(my.px[0], it), p0y = shfl_f(my.py[0], it);
-            const float p1x = shfl_f(my.px[1], it), p1y = shfl_f(my.py[1], it);
-            const float p2x = shfl_f(my.px[2], it), p2y = shfl_f(my.py[2], it);
-            const float z0 = shfl_f(my.z[0], it), z1 = shfl_f(my.z[1], it), z2 = shfl_f(my.z[2], it);
-            const float inv = shfl_f(my.inv, it);
-            uint32_t cov = 0, pix = 0;
-            float z[S];
-#pragma unroll
-            for (int k = 0; k < S; ++k) z[k] = 0.0f;
-            if (p < total) {
-                const uint32_t rr = p - exc;
-                const uint32_t x0 = gg & 31u, y0 = (gg >> 5) & 31u, w = (gg >> 10) & 31u, h = (gg >> 16) & 31u;
-                uint32_t row, col;
-                if (gg & (1u << 21)) {
-                    // last box row whose prefix is <= rr (rows trimmed to nothing are skipped)
-                    row = 0;
-#pragma unroll
-                    for (int st = TS / 2; st > 0; st >>= 1)
-                        if (row + st < h && sm.rpre[it][row + st] <= rr) row += st;
-                    col = sm.rsta[it][row] + (rr - sm.rpre[it][row]);
-                } else {
-                    // w < kTrimMin = 4: rr / w with a multiply (exact for rr < 128)
-                    row = w == 1 ? rr : w == 2 ? (rr >> 1) : ((rr * 43u) >> 7);
-                    col = x0 + (rr - row * w);
+        for (uint32_t gb = 0; gb < rtot; gb += 32) {
+            uint32_t c = 0, sp = 0;
+            {
+                const uint32_t marks = __reduce_or_sync(0xFFFFFFFFu, rstart - gb < 32u ? 1u << (rstart - gb) : 0u);
+                const uint32_t j = sm.rowed[rbefore + __popc(marks & upto)];
+                rbefore += __popc(marks);
+                const float px[3] = {shfl_f(my.px[0], j), shfl_f(my.px[1], j), shfl_f(my.px[2], j)};
+                const float py[3] = {shfl_f(my.py[0], j), shfl_f(my.py[1], j), shfl_f(my.py[2], j)};
+                const bool finite = fabsf(shfl_f(my.inv, j)) <= FLT_MAX;
+                const uint32_t gj = shfl_u(geo, j), rj = shfl_u(rstart, j);
+                if (gb + lane < rtot) {
+                    const uint32_t ly = ((gj >> 8) & 0xFFu) + (gb + lane - rj);
+                    uint32_t a0 = gj & 0xFFu, a1 = gj >> 16;
+                    if (a1 - a0 >= kTrimMin && finite) line_span_pts<S, TS>(px, py, 0u, ly, X0, Y0, a0, a1);
+                    c = a1 - a0;
+                    sp = j | (ly << 8) | (a0 << 16);
                 }
-                const uint32_t ly = y0 + row;
-                pix = ly * TS + col;
-                const float fx = (float)(X0 + col), fy = (float)(Y0 + ly);
-                const Cover<S> cv = cover_pixel<S>(p0x, p0y, p1x, p1y, p2x, p2y, inv, z0, z1, z2, fx, fy);
-                cov = cv.mask;
-#pragma unroll
-                for (int k = 0; k < S; ++k) z[k] = cv.z[k];
             }
-            const uint32_t bal = __ballot_sync(0xFFFFFFFFu, cov != 0);
-            if (cov) {
-                const uint32_t q = (tail + __popc(bal & lanemask_lt())) & (U::QC - 1);
-                sm.qitem[q] = (uint8_t)it;
-                sm.qpix[q] = (uint8_t)pix;
-                sm.qcov[q] = (uint8_t)cov;
-#pragma unroll
-                for (int k = 0; k < S; ++k) sm.qz[k][q] = z[k];
-            }
-            tail += __popc(bal);
+            const uint32_t incl = warp_incl_scan(c);
+            const uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            const uint32_t full = __ballot_sync(0xFFFFFFFFu, c != 0);
+            const uint32_t start = c ? incl - c : 0xFFFFFFFFu;
+            if (c) sm.run[__popc(full & lanemask_lt())] = make_uint2(start, sp);
             __syncwarp();
-            if (tail - head >= 32) {
-                wdepth<S, TS>(sm, my, head, 32, stail, s, X0, Y0, shaded, fsinv);
-                head += 32;
-                if (stail - shead >= 32) {
-                    wshade<S, TS>(sm, my, shead, 32, draws, f, s, X0, Y0, oobc);
-                    shead += 32;
+            // ---- C. the spans' candidates, 32 at a time, in submission order
+            uint32_t before = 0xFFFFFFFFu;  // spans that start in earlier windows, less one
+            for (uint32_t pb = 0; pb < total; pb += 32) {
+                const uint32_t p = pb + lane;
+                const uint32_t marks = __reduce_or_sync(0xFFFFFFFFu, start - pb < 32u ? 1u << (start - pb) : 0u);
+                const uint2 r = sm.run[before + __popc(marks & upto)];
+                before += __popc(marks);
+                const uint32_t it = r.y & 31u;
+                // the item's points, depths and 1 / 2x area from its lane
+                const float p0x = shfl_f(my.px[0], it), p0y = shfl_f(my.py[0], it);
+                const float p1x = shfl_f(my.px[1], it), p1y = shfl_f(my.py[1], it);
+                const float p2x = shfl_f(my.px[2], it), p2y = shfl_f(my.py[2], it);
+                const float z0 = shfl_f(my.z[0], it), z1 = shfl_f(my.z[1], it), z2 = shfl_f(my.z[2], it);
+                const float inv = shfl_f(my.inv, it);
+                uint32_t cov = 0, pix = 0;
+                float z[S];
+#pragma unroll
+                for (int k = 0; k < S; ++k) z[k] = 0.0f;
+                if (p < total) {
+                    const uint32_t ly = (r.y >> 8) & 0xFFu, lx = (r.y >> 16) + (p - r.x);
+                    pix = ly * TS + lx;
+                    const float fx = (float)(X0 + lx), fy = (float)(Y0 + ly);
+                    const Cover<S> cv = cover_pixel<S>(p0x, p0y, p1x, p1y, p2x, p2y, inv, z0, z1, z2, fx, fy);
+                    cov = cv.mask;
+#pragma unroll
+                    for (int k = 0; k < S; ++k) z[k] = ((cov >> k) & 1u) ? cv.z[k] : __int_as_float(0x7FC00000);
+                }
+                const uint32_t bal = __ballot_sync(0xFFFFFFFFu, cov != 0);
+                if (cov) {
+                    const uint32_t q = (tail + __popc(bal & lanemask_lt())) & (U::QC - 1);
+                    sm.q[q] = it | (pix << 8) | (cov << 16);
+                    store_samples<S>(sm.qz[q], z);
+                }
+                tail += __popc(bal);
+                __syncwarp();
+                if (tail - head >= 32) {
+                    wdepth<S, TS>(sm, my, head, 32, stail, s, X0, Y0, shaded, fsinv);
+                    head += 32;
+                    if (stail - shead >= 32) {
+                        wshade<S, TS>(sm, my, shead, 32, draws, f, s, X0, Y0, oobc);
+                        shead += 32;
+                    }
                 }
             }
+            __syncwarp();  // the runs are read before the next group's replace them
         }
         if (tail != head) wdepth<S, TS>(sm, my, head, tail - head, stail, s, X0, Y0, shaded, fsinv);
         while (stail != shead) {
@@ -505,7 +479,7 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const FrameDe
         __syncwarp();
     }
     __syncwarp();
-    wresolve<S, TS>(sm, f, X0, Y0);
+    wresolve<S, TS>(sm, f, X0, Y0, row0, row1);
     __syncwarp();
 }
 
@@ -529,10 +503,15 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 :
     load_queue(sh.tq, queue, order, ntotal, s.status, first_tile);
     const uint32_t nheavy = heavy_tiles(sh.tq, frames[0].heavy_bits);
     const uint32_t nsub = nsx * nsx;
-    const uint32_t nlight = (sh.tq.busy - nheavy) * nsub;
+    // units of the light bins, in strips where they are few. (Strips of the deepest bins, whose length sets
+    // a launch's when it runs alone - 627 -> 519 us for the one-sample scenes of a batch of 20 - cost
+    // 1% where the batch's other launch fills the tail, which a mixed batch always has.)
+    const uint32_t nwhole = (sh.tq.busy - nheavy) * nsub;
+    const uint32_t places = gridDim.x * kWarpUnitWarps;
+    const uint32_t ssh = strips_for(nwhole, places), nlight = nwhole << ssh;
     uint32_t shaded = 0, fsinv = 0, oobc = 0;
     // with no more units than warps, one unit per warp by its place, SMs first (see k_raster)
-    const bool few = nlight <= gridDim.x * kWarpUnitWarps;
+    const bool few = nlight <= places;
     for (bool more = true; more; more = !few) {
         uint32_t qi = warp * gridDim.x + blockIdx.x;
         if (!few) {
@@ -540,7 +519,8 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 :
             qi = __shfl_sync(0xFFFFFFFFu, qi, 0);
         }
         if (qi >= nlight) break;
-        const uint32_t gt = busy_tile(sh.tq, nheavy + qi / nsub), sub = qi % nsub;
+        const uint32_t row0 = (qi & ((1u << ssh) - 1u)) * (TS >> ssh), row1 = row0 + (TS >> ssh);
+        const uint32_t sub = (qi >> ssh) % nsub, gt = busy_tile(sh.tq, nheavy + (qi >> ssh) / nsub);
         const FrameDev& f = frames[frame_of_tile(frames, nframes, gt)];
         const uint32_t lt = gt - f.tile_begin;
         const uint32_t X0 = (lt % f.tiles_x) * (uint32_t)f.ts + (sub % nsx) * TS;
@@ -554,7 +534,7 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 :
             nent = s.tile_count[gt];
             bins = s.bins + f.bin_base + s.tile_start[gt];
         }
-        warp_unit<S, TS>(sm, f, draws, s, bins, nent, 1u << sub, X0, Y0, shaded, fsinv, oobc);
+        warp_unit<S, TS>(sm, f, draws, s, bins, nent, 1u << sub, X0, Y0, row0, row1, shaded, fsinv, oobc);
     }
     // bins without entries: runs of kEmptyRun bins per counter update, the clear colour
     for (;;) {
