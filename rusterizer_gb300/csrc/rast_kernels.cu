@@ -1421,10 +1421,16 @@ __device__ __forceinline__ void warp_depth(RasterSmem<S, TS>& sm, uint32_t w, ui
         load_samples<S>(sm.qz[w][q], z);
     }
     const uint32_t pix = (fr >> 8) & 0xFFu;
-    const uint32_t key = valid ? pix : 0x10000u + lane;
-    const uint32_t grp = __match_any_sync(0xFFFFFFFFu, key);
-    const uint32_t rank = __popc(grp & lanemask_lt());
-    const uint32_t maxr = __reduce_max_sync(0xFFFFFFFFu, rank);
+    // fragments of one item never share a pixel: most windows over large triangles need no match, whose
+    // time grows with the distinct values (3 000 large triangles at 1440p 473 -> 460 us a frame; no
+    // change on the soups, 0.3% on the 2M-triangle terrain, whose windows mix items)
+    uint32_t rank = 0, maxr = 0;
+    const uint32_t fr0 = __shfl_sync(0xFFFFFFFFu, fr, 0);  // every lane
+    if (!__all_sync(0xFFFFFFFFu, (!valid) | (((fr ^ fr0) & 0xFFu) == 0))) {
+        const uint32_t key = valid ? pix : 0x10000u + lane;
+        rank = __popc(__match_any_sync(0xFFFFFFFFu, key) & lanemask_lt());
+        maxr = __reduce_max_sync(0xFFFFFFFFu, rank);
+    }
     uint32_t dm = 0;
     for (uint32_t r = 0; r <= maxr; ++r) {
         // this round's lanes: no two share a pixel
