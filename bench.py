@@ -39,11 +39,11 @@ AUTO_BIG_BIN_TRIS = 8192  # from this many triangles the library picks 32-pixel 
 
 
 def launches_per_frame(width, height, ntris, tile=0):
-    """Kernels per plain frame: vertex, bin count, clip, column scan, tile scan (which also
-    builds the raster tile queue of a one-frame run), scatter, raster, plus the quadrant split
-    when the frame uses 32-pixel bins (the library's automatic choice: 32-pixel bins for frames
-    of AUTO_BIG_BIN_TRIS triangles or more, else 16, either one when the other would exceed
-    COUNT_BAND_TILES bins, and 32 for frames where both would)."""
+    """8 where a plain frame uses 32-pixel bins, else 7: the library's automatic choice is 32-pixel
+    bins for frames of AUTO_BIG_BIN_TRIS triangles or more, else 16, either one when the other would
+    exceed COUNT_BAND_TILES bins, and 32 for frames where both would. (The numbers are the launches of
+    the pipeline with a tile scan of its own; it takes one fewer now, and 3 for small frames. What
+    a run launches is counted: gpu_launches.)"""
     def bins(t):
         return -(-width // t) * -(-height // t)
     if not (tile in (8, 16, 32) and bins(tile) <= MAX_TILES_PER_FRAME):

@@ -4,7 +4,8 @@
 // pipeline (grown on demand and kept across frames), a pinned staging area for the per-frame
 // descriptors, and a small device state block (status bits, statistics, allocation counters).
 // A frame is one descriptor upload (skipped when the descriptors are unchanged), one state
-// reset, seven kernel launches (eight with 32-pixel bins) and one state readback; capacity
+// reset, six kernel launches (seven with 32-pixel bins, three for a small frame) and one state
+// readback; capacity
 // overflows (bins, clip store) are detected on the device and the frame is re-run with the
 // measured sizes (at most twice). rast_framebuffer_async skips the readback; into host memory it
 // resolves into alternating staging buffers that a side stream copies out.

@@ -1,6 +1,6 @@
 // rast_kernels.cu - sm_103a kernels of the raster pipeline.
 //
-//   k_vertex       per vertex: MVP * v, divide, viewport, clip predicates       (HBM-bound)
+//   k_vertex       per vertex: MVP * v, divide, viewport; one word for binning  (HBM-bound)
 //   k_bin_count    per chunk of triangles: classify, tile rectangle, per-chunk tile histogram
 //                  in shared memory (band by band for frames of more than 16384 bins)
 //   k_clip         one warp per triangle that straddles a clip plane: clip, fan boxes, counts
@@ -381,8 +381,8 @@ __global__ void __launch_bounds__(256, 6) k_bin_count(const ChunkDev* __restrict
     pdl_enter();
     // per-bin counts of the chunk, two 16-bit counters per word (bin t in half t & 1 of word
     // t / 2): a chunk holds at most 8192 triangles, so no counter carries into its neighbour,
-    // and the histogram of kCountBandTiles = 16384 bins takes 32 KB (six CTAs per SM: registers, 0.99 of the frame time of eight; room for seven for the
-    // largest frames). Frames with more bins are counted band by band: the first pass
+    // and the histogram of kCountBandTiles = 16384 bins takes 32 KB (6 CTAs per SM by registers: 431 us
+    // a frame against 436 with 8 on the 2M-triangle terrain). Frames with more bins are counted band by band: the first pass
     // classifies the triangles and stores their boxes, later passes read the boxes back and
     // count the bins of their band (rows of the box outside the band are skipped).
     extern __shared__ uint32_t hist[];

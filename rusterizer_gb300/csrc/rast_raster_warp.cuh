@@ -4,7 +4,7 @@
 // partial warps between block barriers. Here one warp owns a whole tile: it stages the tile's
 // items 32 at a time, one per lane and held in that lane's registers (other lanes read them
 // with shuffles, which keeps shared memory for the samples and rings: 5 CTAs of 4 warps per
-// SM with four samples per pixel, 6 with one), walks their candidate pixels 32 at a time, depth-tests the covered fragments in
+// SM), walks their candidate pixels 32 at a time, depth-tests the covered fragments in
 // submission order and shades the passed ones, with full warps and no block barrier. The
 // arithmetic is the same device functions as k_raster (coverage, sample depths, tie rule,
 // interpolation, shaders, resolve), so results are bit-identical; only the work split differs.
@@ -302,7 +302,7 @@ __device__ __forceinline__ void wresolve(const WarpUnitSmem<S, TS>& sm, const Fr
     }
 }
 
-// One light tile by one warp: the bin's entries in submission order, 32 items at a time.
+// One light tile (or strip of its rows) by one warp: the entries in submission order, 32 items at a time.
 // (A) the items of the next entries, one per lane (a lane finds its entry and fan triangle
 // from the entries' running item counts); (B) per item (lane) its candidate pixels: the whole
 // tile-local box, or for boxes of kTrimMin+ columns each row trimmed by line_span; (C) the
