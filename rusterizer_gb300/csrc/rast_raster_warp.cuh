@@ -145,10 +145,15 @@ __device__ __forceinline__ void wdepth(WarpUnitSmem<S, TS>& sm, const WItem& my,
         lmeta = shfl_u(my.meta, fr & 31u);
     }
     const uint32_t pix = (fr >> 8) & 0xFFu;
-    const uint32_t key = valid ? pix : 0x10000u + lane;
-    const uint32_t grp = __match_any_sync(0xFFFFFFFFu, key);
-    const uint32_t rank = __popc(grp & lanemask_lt());
-    const uint32_t maxr = __reduce_max_sync(0xFFFFFFFFu, rank);
+    // windows of one item need no match (see warp_depth): a captured batch of 20 scenes 1160 -> 1105 us,
+    // with the same test in the shader
+    uint32_t rank = 0, maxr = 0;
+    const uint32_t fr0 = __shfl_sync(0xFFFFFFFFu, fr, 0);  // every lane
+    if (!__all_sync(0xFFFFFFFFu, (!valid) | (((fr ^ fr0) & 0xFFu) == 0))) {
+        const uint32_t key = valid ? pix : 0x10000u + lane;
+        rank = __popc(__match_any_sync(0xFFFFFFFFu, key) & lanemask_lt());
+        maxr = __reduce_max_sync(0xFFFFFFFFu, rank);
+    }
     uint32_t dm = 0;
     for (uint32_t r = 0; r <= maxr; ++r) {
         if (valid && rank == r) {
@@ -240,10 +245,13 @@ __device__ __forceinline__ void wshade(WarpUnitSmem<S, TS>& sm, const WItem& my,
             argb = to_argb(col[0], col[1], col[2], col[3]);
         }
     }
-    const uint32_t key = valid ? pix : 0x10000u + lane;
-    const uint32_t grp = __match_any_sync(0xFFFFFFFFu, key);
-    const uint32_t rank = __popc(grp & lanemask_lt());
-    const uint32_t maxr = __reduce_max_sync(0xFFFFFFFFu, rank);
+    uint32_t rank = 0, maxr = 0;  // windows of one item need no match, as in wdepth
+    const uint32_t it0 = __shfl_sync(0xFFFFFFFFu, it, 0);  // every lane
+    if (!__all_sync(0xFFFFFFFFu, (!valid) | (it == it0))) {
+        const uint32_t key = valid ? pix : 0x10000u + lane;
+        rank = __popc(__match_any_sync(0xFFFFFFFFu, key) & lanemask_lt());
+        maxr = __reduce_max_sync(0xFFFFFFFFu, rank);
+    }
     for (uint32_t r = 0; r <= maxr; ++r) {
         const bool act = valid && rank == r;
 #pragma unroll
