@@ -220,11 +220,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
             E.desc_bytes = total;
             E.d_desc_ptr = E.d_desc.p;
         }
-        // the state block: k_vertex clears it, or a memset where the first kernel uses it (k_front) or
-        // there are no vertices
-        const bool clear = small || vblocks.empty();
-        if (clear && cudaMemsetAsync(E.d_state, 0, Engine::state_bytes(frames.size()), st) != cudaSuccess)
-            return RAST_CUDA_ERROR;
+        if (cudaMemsetAsync(E.d_state, 0, Engine::state_bytes(frames.size()), st) != cudaSuccess) return RAST_CUDA_ERROR;
 
         LaunchArgs a{};
         a.stream = st;
@@ -235,8 +231,6 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         a.nchunks = (uint32_t)chunks.size();
         a.vblocks = reinterpret_cast<const uint2*>(E.d_desc.p + off_vblocks);
         a.vertex_blocks = (uint32_t)vblocks.size();
-        a.state = reinterpret_cast<uint32_t*>(E.d_state);
-        a.state_words = clear ? 0u : (uint32_t)(Engine::state_bytes(frames.size()) / 4);
         a.scan_groups = group_tot;
         a.max_tiles = max_tiles;
         Scratch& S = a.scratch;

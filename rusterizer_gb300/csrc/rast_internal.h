@@ -176,7 +176,7 @@ struct FrameJob {
     uint64_t need = 0;       // bins the frame used (filled after a synchronous run)
 };
 
-// Device state block cleared at the start of every launch sequence (k_vertex or a memset); the frames' bin allocation
+// Device state block reset at the start of every launch sequence; the frames' bin allocation
 // counters (Scratch::frame_need) follow it in the same buffer.
 struct DeviceState {
     uint32_t status;

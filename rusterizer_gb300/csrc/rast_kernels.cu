@@ -140,16 +140,10 @@ __device__ __forceinline__ float4 vertex_bin(float4 c, float4 sc) {
     return make_float4((code & kInsideAll) == kInsideAll ? c.x : __uint_as_float(kVbinTag | code), c.y, sc.x, sc.y);
 }
 
-// The first CTA also clears the run's state block, `state_words` words that no vertex CTA reads or writes
-// (the kernels after this one do): a memset of its own in front kept this kernel from being scheduled
-// beside the end of the frame before (100k soup 286.6 -> 284.4 us a frame, 500k terrain 554 -> 547 for two).
 __global__ void __launch_bounds__(256) k_vertex(const DrawDev* __restrict__ draws,
                                                 const FrameDev* __restrict__ frames,
-                                                const uint2* __restrict__ vblocks, uint32_t* __restrict__ state,
-                                                uint32_t state_words, Scratch s) {
+                                                const uint2* __restrict__ vblocks, Scratch s) {
     pdl_enter();
-    if (blockIdx.x == 0)
-        for (uint32_t i = threadIdx.x; i < state_words; i += blockDim.x) state[i] = 0;
     const uint2 vb = vblocks[blockIdx.x];
     const DrawDev& d = draws[vb.x];
     const uint32_t v = vb.y + threadIdx.x;
@@ -388,8 +382,8 @@ __global__ void __launch_bounds__(256, 6) k_bin_count(const ChunkDev* __restrict
     // per-bin counts of the chunk, two 16-bit counters per word (bin t in half t & 1 of word
     // t / 2): a chunk holds at most 8192 triangles, so no counter carries into its neighbour,
     // and the histogram of kCountBandTiles = 16384 bins takes 32 KB (6 CTAs per SM by registers: 431 us
-    // a frame against 436 with 8 on the 2M-triangle terrain). Frames with more bins are counted band
-    // by band: the first pass classifies the triangles and stores their boxes, later passes read the boxes back and
+    // a frame against 436 with 8 on the 2M-triangle terrain). Frames with more bins are counted band by band: the first pass
+    // classifies the triangles and stores their boxes, later passes read the boxes back and
     // count the bins of their band (rows of the box outside the band are skipped).
     extern __shared__ uint32_t hist[];
     const ChunkDev ch = chunks[blockIdx.x];
@@ -897,8 +891,7 @@ static_assert(kGatherTris % 32 == 0 && kGatherTris / 32 < 256, "a lane's entries
 __global__ void __launch_bounds__(kGatherThreads) k_bin_gather(const FrameDev* __restrict__ frames, int nframes,
                                                                Scratch s) {
     pdl_enter();
-    // by triangle: its bins of the block, x0 | x1 << 3 | y0 << 6 | y1 << 9 | clipped << 15
-    __shared__ uint16_t abox[kGatherTris];
+    __shared__ uint16_t abox[kGatherTris];  // by triangle: bins of the block x0 | x1 << 3 | y0 << 6 | y1 << 9 | clipped << 15
     __shared__ uint16_t ltri[kGatherTris];  // the block's triangles in order
     __shared__ uint32_t hit[kGatherTris / 32];
     __shared__ uint32_t wcount[kGatherWarps];
@@ -2105,8 +2098,7 @@ static cudaError_t launch_raster_t(const LaunchArgs& a, uint32_t nsx) {
 
 cudaError_t launch_vertex(const LaunchArgs& a) {
     if (a.vertex_blocks == 0) return cudaSuccess;
-    return launch_pdl(k_vertex, a.vertex_blocks, 256, 0, a.stream, a.draws, a.frames, a.vblocks, a.state,
-                      a.state_words, a.scratch);
+    return launch_pdl(k_vertex, a.vertex_blocks, 256, 0, a.stream, a.draws, a.frames, a.vblocks, a.scratch);
 }
 
 cudaError_t launch_front(const LaunchArgs& a) {

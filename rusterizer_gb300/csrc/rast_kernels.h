@@ -18,8 +18,6 @@ struct LaunchArgs {
     uint32_t nchunks;
     const uint2* vblocks;  // (draw, first vertex) per 256-vertex block
     uint32_t vertex_blocks;
-    uint32_t* state;         // the state block that launch_vertex clears (state_words 0: cleared before)
-    uint32_t state_words;
     uint32_t scan_groups;  // scan groups over all frames
     uint32_t max_tiles;    // largest per-frame tile count
     // raster launch over one (msaa, tile) group of consecutive frames
