@@ -382,8 +382,8 @@ __global__ void __launch_bounds__(256, 6) k_bin_count(const ChunkDev* __restrict
     // per-bin counts of the chunk, two 16-bit counters per word (bin t in half t & 1 of word
     // t / 2): a chunk holds at most 8192 triangles, so no counter carries into its neighbour,
     // and the histogram of kCountBandTiles = 16384 bins takes 32 KB (6 CTAs per SM by registers: 431 us
-    // a frame against 436 with 8 on the 2M-triangle terrain). Frames with more bins are counted band by band: the first pass
-    // classifies the triangles and stores their boxes, later passes read the boxes back and
+    // a frame against 436 with 8 on the 2M-triangle terrain). Frames with more bins are counted band
+    // by band: the first pass classifies the triangles and stores their boxes, later passes read the boxes back and
     // count the bins of their band (rows of the box outside the band are skipped).
     extern __shared__ uint32_t hist[];
     const ChunkDev ch = chunks[blockIdx.x];
