@@ -846,6 +846,8 @@ __global__ void __launch_bounds__(256) k_front(const ChunkDev* __restrict__ chun
         sv[q] = make_float4(__shfl_sync(0xFFFFFFFFu, sc.x, q0 + q), __shfl_sync(0xFFFFFFFFu, sc.y, q0 + q), 0.0f, 0.0f);
     }
     const uint32_t g0 = f.rect_base + d.tbase + tri0;
+    // each triangle's words have one writer: lane t here, or lane 0 for a straddler below (nothing in
+    // between orders two lanes' stores to one address)
     bool straddles = false;
     if (lane < nt) {
         unsigned long long rect = kRectEmpty;
@@ -860,8 +862,10 @@ __global__ void __launch_bounds__(256) k_front(const ChunkDev* __restrict__ chun
             }
             straddles = cls == 2;
         }
-        s.tri_rect[g0 + lane * nw] = rect;
-        s.tri_aux[g0 + lane * nw] = kNone;
+        if (!straddles) {
+            s.tri_rect[g0 + lane * nw] = rect;
+            s.tri_aux[g0 + lane * nw] = kNone;
+        }
     }
     for (uint32_t m = __ballot_sync(0xFFFFFFFFu, straddles); m; m &= m - 1) {
         const uint32_t t = __ffs(m) - 1, src = min(3 * t + lane, 31u);
@@ -870,9 +874,10 @@ __global__ void __launch_bounds__(256) k_front(const ChunkDev* __restrict__ chun
                                       __shfl_sync(0xFFFFFFFFu, c.z, src), __shfl_sync(0xFFFFFFFFu, c.w, src));
         uint32_t off = 0;
         const unsigned long long rect = clip_triangle(d, f, s, cvi, cc, off);
-        if (rect != kRectEmpty && lane == 0) {
-            s.tri_rect[g0 + t * nw] = rect | kRectClippedBit;
-            s.tri_aux[g0 + t * nw] = off;
+        if (lane == 0) {
+            const bool gone = rect == kRectEmpty;
+            s.tri_rect[g0 + t * nw] = gone ? kRectEmpty : rect | kRectClippedBit;
+            s.tri_aux[g0 + t * nw] = gone ? kNone : off;
         }
         __syncwarp();
     }
