@@ -76,11 +76,14 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
     E.h_order = order;
     // every frame small: the front and gather kernels (see k_bin_gather)
     bool small = true;
+    uint64_t run_tris = 0;
     for (const FrameJob& J : jobs) {
         uint64_t t = 0;
         for (const DrawJob& DJ : J.draws) t += DJ.mesh->ntris;
         small = small && t <= kGatherTris;
+        run_tris += t;
     }
+    const uint32_t per_warp = front_tris(run_tris);
 
     for (int attempt = 0; attempt < 3; ++attempt) {
         std::vector<FrameDev>& frames = E.h_frames;
@@ -132,7 +135,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
                 const uint32_t di = (uint32_t)draws.size();
                 draws.push_back(D);
                 for (uint32_t v = 0; v < m->nverts; v += 256) vblocks.push_back(make_uint2(di, v));
-                const uint32_t cs = small ? kGatherChunk : chunk_size_for(std::max<uint32_t>(J.ntris_hint, m->ntris));
+                const uint32_t cs = small ? 8 * per_warp : chunk_size_for(std::max<uint32_t>(J.ntris_hint, m->ntris));
                 for (uint32_t t = 0; t < m->ntris; t += cs) {
                     ChunkDev C{};
                     C.draw = di;
@@ -231,6 +234,7 @@ rast_status run_frames(Engine& E, std::vector<FrameJob>& jobs) {
         a.nchunks = (uint32_t)chunks.size();
         a.vblocks = reinterpret_cast<const uint2*>(E.d_desc.p + off_vblocks);
         a.vertex_blocks = (uint32_t)vblocks.size();
+        a.front_tris = per_warp;
         a.scan_groups = group_tot;
         a.max_tiles = max_tiles;
         Scratch& S = a.scratch;

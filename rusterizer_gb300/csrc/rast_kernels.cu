@@ -788,20 +788,17 @@ __global__ void __launch_bounds__(kScatterThreads) k_bin_scatter(
 // no longer fit shared memory, and the chunks begin to fill the GPU (8 000 small terrain triangles
 // on 640x480 are the one case that the chunk path does better: 54 against 60 us).
 
-constexpr int kFrontTris = 4;                            // triangles per warp of k_front
-constexpr int kFrontChunk = 8 * kFrontTris;              // per CTA
-static_assert(kFrontChunk == (int)kGatherChunk, "chunks of small frames are one CTA of k_front");
-
 // The first vertex_blocks CTAs transform 256 vertices each (what the raster reads: screen points); the
-// others take a chunk of kFrontChunk triangles, kFrontTris per warp: lane 3 t + q transforms corner
-// q of triangle t again from its position (no wait for the vertex CTAs), lane t classifies triangle t,
-// and the whole warp clips the ones that straddle a plane, one after another. Few triangles per
-// warp, from as many places of the mesh, keep that chain short: a mesh may hold all its
-// straddlers in a row (2 000 triangles, 200 straddlers: 13 us with four neighbours per warp, 9 spread).
+// others take a chunk of 8 `per` triangles, `per` (front_tris: 4, or 10 in a run of many) of them to a
+// warp: lane 3 t + q transforms corner q of triangle t again from its position (no wait for the
+// vertex CTAs), lane t classifies triangle t, and the whole warp clips the ones that straddle a plane, one
+// after another. Few triangles per warp, from as many places of the mesh, keep that chain short: a mesh may hold all
+// its straddlers in a row (2 000 triangles, 200 straddlers: 13 us with four neighbours per warp, 9 spread).
 __global__ void __launch_bounds__(256) k_front(const ChunkDev* __restrict__ chunks,
                                                const DrawDev* __restrict__ draws,
                                                const FrameDev* __restrict__ frames,
-                                               const uint2* __restrict__ vblocks, uint32_t vertex_blocks, Scratch s) {
+                                               const uint2* __restrict__ vblocks, uint32_t vertex_blocks,
+                                               uint32_t per, Scratch s) {
     pdl_enter();
     if (blockIdx.x < vertex_blocks) {
         const uint2 vb = vblocks[blockIdx.x];
@@ -817,10 +814,10 @@ __global__ void __launch_bounds__(256) k_front(const ChunkDev* __restrict__ chun
     const FrameDev& f = frames[d.frame];
     const uint32_t lane = lane_id();
     // triangle t of this warp: tri0 + t * nw, nw warps in the draw
-    const uint32_t nw = (d.ntris + kFrontTris - 1) / kFrontTris;
-    const uint32_t tri0 = ch.tri_begin / kFrontTris + (threadIdx.x >> 5);
+    const uint32_t nw = (d.ntris + per - 1) / per;
+    const uint32_t tri0 = ch.tri_begin / per + (threadIdx.x >> 5);
     if (tri0 >= nw) return;  // whole warps
-    const uint32_t nt = min((uint32_t)kFrontTris, (d.ntris - tri0 + nw - 1) / nw);
+    const uint32_t nt = min(per, (d.ntris - tri0 + nw - 1) / nw);
     uint32_t vi = 0, code = 0;
     bool bad = false;
     float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f), sc = c;
@@ -2182,7 +2179,7 @@ cudaError_t launch_vertex(const LaunchArgs& a) {
 cudaError_t launch_front(const LaunchArgs& a) {
     if (a.vertex_blocks + a.nchunks == 0) return cudaSuccess;
     return launch_pdl(k_front, a.vertex_blocks + a.nchunks, 256, 0, a.stream, a.chunks, a.draws, a.frames, a.vblocks,
-                      a.vertex_blocks, a.scratch);
+                      a.vertex_blocks, a.front_tris, a.scratch);
 }
 
 cudaError_t launch_gather(const LaunchArgs& a) {

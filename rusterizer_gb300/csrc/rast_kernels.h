@@ -18,6 +18,7 @@ struct LaunchArgs {
     uint32_t nchunks;
     const uint2* vblocks;  // (draw, first vertex) per 256-vertex block
     uint32_t vertex_blocks;
+    uint32_t front_tris;   // small runs: triangles per warp of k_front (a chunk holds 8 times that)
     uint32_t scan_groups;  // scan groups over all frames
     uint32_t max_tiles;    // largest per-frame tile count
     // raster launch over one (msaa, tile) group of consecutive frames

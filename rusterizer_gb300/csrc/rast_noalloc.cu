@@ -29,6 +29,7 @@ namespace {
 constexpr size_t kNoAllocScratchBytes = size_t(32) << 20;
 constexpr uint32_t kNoAllocMaxVerts = 262144;
 constexpr uint32_t kNoAllocMaxTris = 262144;
+constexpr uint32_t kOneFrameFront = rast::front_tris(rast::kGatherTris);
 constexpr uint32_t kMinChunk = 256;  // smallest chunk chunk_size_for returns
 constexpr int kMaxDevices = 64;
 
@@ -145,7 +146,7 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
     const uint32_t big_chunks = (ntris + big_cs - 1) / big_cs;
     const uint32_t nvb = (nverts + 255u) / 256u;
     // chunk_size_for never goes below kMinChunk, so the descriptor arrays always hold them
-    static_assert((kGatherTris + kGatherChunk - 1) / kGatherChunk <= sizeof(g_chunks) / sizeof(g_chunks[0]),
+    static_assert((kGatherTris + 8 * kOneFrameFront - 1) / (8 * kOneFrameFront) <= sizeof(g_chunks) / sizeof(g_chunks[0]),
                   "the staging array holds a small frame's chunks");
     if (big_cs < kMinChunk || big_chunks > sizeof(g_chunks) / sizeof(g_chunks[0]) ||
         nvb > sizeof(g_vblocks) / sizeof(g_vblocks[0]))
@@ -198,7 +199,7 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
         // the general path
         F.order_coarse = 0;
         bool small = ntris <= kGatherTris;
-        uint32_t cs = small ? kGatherChunk : big_cs, nchunks = (ntris + cs - 1) / cs;
+        uint32_t cs = small ? 8 * kOneFrameFront : big_cs, nchunks = (ntris + cs - 1) / cs;
         Layout L = carve_layout(nverts, ntris, nchunks, big_chunks, nvb, F.ntiles, split, bin_cap, clip_floats, false);
         if (L.end > kNoAllocScratchBytes) {
             F.order_coarse = 1;
@@ -246,6 +247,7 @@ extern "C" rast_status rast_render_noalloc(int width, int height, int msaa, int 
         a.nchunks = nchunks;
         a.vblocks = reinterpret_cast<const uint2*>(base + L.vblocks);
         a.vertex_blocks = nvb;
+        a.front_tris = kOneFrameFront;
         a.scan_groups = small ? gather_groups(F.tiles_x, F.tiles_y, F.gather_bins) : (F.ntiles + 31) / 32;
         a.max_tiles = F.ntiles;
         a.raster_frames = a.frames;
