@@ -87,6 +87,21 @@ inline uint32_t gather_edge(uint32_t tiles_x, uint32_t tiles_y) {
     return gather_groups(tiles_x, tiles_y, 8) >= 100 ? 8 : 4;
 }
 
+// Device bytes that a one-draw frame of width x height with bins of edge ts takes while in flight (what
+// run_frames reserves for it, and its image): vertex records, per-triangle boxes and straddler list, chunk
+// histograms, bin tables and raster queue, bins (and quadrant lists for 32-pixel bins), clip store. `bins`:
+// entries that an earlier such frame needed.
+inline uint64_t frame_bytes(uint64_t nverts, uint32_t ntris, uint64_t width, uint64_t height, int ts, uint64_t bins) {
+    const uint64_t tiles = ((width + ts - 1) / ts) * ((height + ts - 1) / ts);
+    const uint64_t cs = chunk_size_for(ntris), chunks = (ntris + cs - 1) / cs;
+    const uint64_t first = 4ull * ntris + tiles + 1024ull, cap = bins > first ? bins : first;
+    const uint64_t split = raster_edge(ts) < ts ? 16ull * (cap + tiles) : 0ull;       // qbins, qcount
+    return 2ull * 16 * nverts                                                          // vbin, vscr
+           + (8ull + 4 + 12) * ntris                                                   // tri_rect, tri_aux, clip_list
+           + 4ull * chunks * tiles + 4ull * (2 + kOrderArrays) * tiles                 // counts; start, count, order
+           + 4ull * cap + split + 4ull * (32ull * ntris + 4096) + 4ull * width * height + 65536ull;
+}
+
 enum StatusBits : uint32_t {
     ST_TEXTURE_OOB = 1u << 0,
     ST_BIN_OVERFLOW = 1u << 1,
