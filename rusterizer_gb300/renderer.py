@@ -173,9 +173,10 @@ class Renderer:
                                            rg, idx.ctypes.data_as(_u32p)), "mesh update")
 
     def update_async(self, mesh, pos, uv, idx, rgba=None):
-        """Like update(), with the copies on a side stream after the frames already enqueued; the
-        next frame that draws this mesh waits for them on the device. The arrays must stay
-        unchanged until that frame is done (page-locked arrays make the copies asynchronous)."""
+        """Like update(), with the copies on a side stream after the frames already enqueued that
+        draw this mesh, beside frames of other meshes; the next frame that draws it waits for them on
+        the device. The arrays must stay unchanged until that frame is done (page-locked arrays
+        make the copies asynchronous)."""
         h = self.upload(mesh)
         ptr = lambda a: ctypes.cast(_data_ptr(a), _fp)  # noqa: E731
         check(_lib.load().rast_mesh_update_async(self._ctx, h, ptr(pos), ptr(uv),
