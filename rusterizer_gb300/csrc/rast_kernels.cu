@@ -436,22 +436,6 @@ __global__ void __launch_bounds__(256, 6) k_bin_count(const ChunkDev* __restrict
 
 // ===================================================================== binning: scans
 
-// Class of a bin in its raster queue by the bit length of its entry count: 0 without entries, then
-// steps at 1, 4, 16, 32, 64, ... 4096 entries; the step nearest to the heavy limit 2^heavy_bits is
-// moved onto it where none lies there, so that the heavy bins are whole classes (heavy_class and up).
-// Steps of 2 where most bins lie: the queue's end is then filled with small tiles (steps of 4 made the
-// 100k-triangle soup at 1080p 3% slower).
-__device__ __forceinline__ uint32_t order_class(uint32_t count, uint32_t heavy_bits) {
-    const uint32_t b = 32 - __clz(count), h = heavy_bits + 1;
-    const uint32_t s2 = h == 2 ? 2u : 3u, s3 = h == 4 ? 4u : 5u, s11 = h >= 13 && h <= 31 ? h : 13u;
-    if (b >= 5) return b >= s11 ? 11u : min(b, 12u) - 2u;
-    return (b >= 1) + (b >= s2) + (b >= s3);
-}
-// Lowest class whose bins are rastered CTA-wide.
-__device__ __forceinline__ uint32_t heavy_class(uint32_t heavy_bits) {
-    const uint32_t h = heavy_bits + 1;
-    return h >= 32 ? (uint32_t)kClasses : h >= 13 ? 11u : h >= 5 ? h - 2u : h >= 4 ? 3u : h >= 2 ? 2u : 1u;
-}
 // Place of the k-th bin of class c in the group's arrays of n tiles: two classes share an array and
 // grow towards each other from its ends.
 __device__ __forceinline__ unsigned long long order_slot(uint32_t c, uint32_t k, uint32_t n) {

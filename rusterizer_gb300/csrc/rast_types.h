@@ -23,6 +23,12 @@
 
 #include <cstdint>
 
+#ifdef __CUDACC__
+#define RAST_HD __host__ __device__
+#else
+#define RAST_HD
+#endif
+
 namespace rast {
 
 constexpr uint32_t kClearColor = 0xFF191919u;  // src/rasterizer/buffers.rs:5
@@ -45,6 +51,26 @@ constexpr int kQueueClass = 4;
 constexpr int kClasses = 12;
 constexpr int kOrderArrays = kClasses / 2;  // arrays of tiles per raster group
 constexpr int kMaxRasterGroups = 8;
+// Class of a bin in its raster queue by the bit length of its entry count: 0 without entries, then
+// steps at 1, 4, 16, 32, 64, ... 4096 entries; the step nearest to the heavy limit 2^heavy_bits is
+// moved onto it where none lies there, so that the heavy bins are whole classes (heavy_class and up).
+// Steps of 2 where most bins lie: the queue's end is then filled with small tiles (steps of 4 made the
+// 100k-triangle soup at 1080p 3% slower).
+RAST_HD inline uint32_t order_class(uint32_t count, uint32_t heavy_bits) {
+#ifdef __CUDA_ARCH__
+    const uint32_t b = 32 - __clz(count), h = heavy_bits + 1;
+#else
+    const uint32_t b = count ? 32u - (uint32_t)__builtin_clz(count) : 0u, h = heavy_bits + 1;
+#endif
+    const uint32_t s2 = h == 2 ? 2u : 3u, s3 = h == 4 ? 4u : 5u, s11 = h >= 13 && h <= 31 ? h : 13u;
+    if (b >= 5) return b >= s11 ? 11u : (b < 12u ? b : 12u) - 2u;
+    return (b >= 1) + (b >= s2) + (b >= s3);
+}
+// Lowest class whose bins are rastered CTA-wide.
+RAST_HD inline uint32_t heavy_class(uint32_t heavy_bits) {
+    const uint32_t h = heavy_bits + 1;
+    return h >= 32 ? (uint32_t)kClasses : h >= 13 ? 11u : h >= 5 ? h - 2u : h >= 4 ? 3u : h >= 2 ? 2u : 1u;
+}
 // Bins with at least 2^kDefaultHeavyBits entries are rastered CTA-wide, the others one warp per
 // raster tile (rast_set_heavy_tile_entries)
 constexpr uint32_t kDefaultHeavyBits = 0;
@@ -55,10 +81,7 @@ constexpr uint32_t kMaxFrameTris = 1u << (32 - kEntShift);
 
 // Edge of the raster tile that one CTA owns for bins of edge ts: 32-pixel bins are rastered as
 // four 16-pixel quadrants (more, smaller units balance the persistent raster kernel better).
-#ifdef __CUDACC__
-__host__ __device__
-#endif
-constexpr int raster_edge(int ts) { return ts > 16 ? 16 : ts; }
+RAST_HD constexpr int raster_edge(int ts) { return ts > 16 ? 16 : ts; }
 
 // Triangles per binning chunk (one CTA of the count and scatter kernels; one row of per-tile
 // counts): about 900 chunks for large meshes, a multiple of 256 in [256, 8192].
