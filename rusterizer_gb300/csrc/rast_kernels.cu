@@ -2251,7 +2251,7 @@ __global__ void k_kat(int op, const unsigned char* __restrict__ in, unsigned cha
     float* fo = reinterpret_cast<float*>(out);
     uint32_t* uo = reinterpret_cast<uint32_t*>(out);
     const int32_t* ii = reinterpret_cast<const int32_t*>(in);
-    if (op != 5 && threadIdx.x != 0) return;
+    if (op != 5 && op != 11 && threadIdx.x != 0) return;
     switch (op) {
         case 0: {  // perspective divide of 3 clip vertices
             for (int v = 0; v < 3; ++v) {
@@ -2369,7 +2369,7 @@ __global__ void k_kat(int op, const unsigned char* __restrict__ in, unsigned cha
             uo[0] = to_argb(fi[0], fi[1], fi[2], fi[3]);
             break;
         }
-        case 9: {  // texture sample: in {i32 w, i32 h, f32 u, f32 v, u32 texels[w*h]}; out {f32[4], u32 oob}
+        case 9: {  // texture sample (tex_argb's way for coordinates outside the texture): in {i32 w, i32 h, f32 u, f32 v, u32 texels[w*h]}; out {f32[4], u32 oob}
             bool oob = false;
             tex_sample(reinterpret_cast<const uint32_t*>(in) + 4, (uint32_t)ii[0], (uint32_t)ii[1], fi[2], fi[3],
                        fo, oob);
@@ -2380,13 +2380,26 @@ __global__ void k_kat(int op, const unsigned char* __restrict__ in, unsigned cha
             for (int r = 0; r < 4; ++r) fo[r] = dot4(fi + 4 * r, fi[16], fi[17], fi[18], fi[19]);
             break;
         }
+        case 11: {  // the shader's texture filter: in {u32 w, h, n, 0, f32 uv[2n], u32 texels[w*h]}; out {u32 argb[n], u32 oob[n]}
+            const uint32_t* ui = reinterpret_cast<const uint32_t*>(in);
+            const uint32_t n = ui[2];
+            DrawDev d;
+            d.set_texture(ui + 4 + 2ull * n, ui[0], ui[1]);
+            for (uint32_t i = threadIdx.x; i < n; i += 32) {
+                uint32_t oob = 0;
+                uo[i] = tex_argb(d.tex, d.tex_w, d.tex_h, d.tex_xmax, d.tex_ymax, d.tex_small != 0, fi[4 + 2 * i],
+                                 fi[5 + 2 * i], true, oob);
+                uo[n + i] = oob;
+            }
+            break;
+        }
         default:
             break;
     }
 }
 
 cudaError_t launch_kat(int op, const void* in, void* out, cudaStream_t stream) {
-    // one warp: op 5 (the warp clipper) uses every lane, the others run on lane 0
+    // one warp: ops 5 (the warp clipper) and 11 use every lane, the others run on lane 0
     k_kat<<<1, 32, 0, stream>>>(op, static_cast<const unsigned char*>(in), static_cast<unsigned char*>(out));
     return cudaGetLastError();
 }

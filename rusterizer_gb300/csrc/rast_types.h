@@ -159,7 +159,7 @@ struct alignas(16) DrawDev {
     uint32_t frame;
     float mvp[16];         // (P * V) * W, row-major
 
-    void set_texture(const uint32_t* data, uint32_t w, uint32_t h) {
+    RAST_HD void set_texture(const uint32_t* data, uint32_t w, uint32_t h) {
         tex = data;
         tex_w = w;
         tex_h = h;
