@@ -38,18 +38,22 @@ MAX_TILES_PER_FRAME = 1 << 22  # the library's per-frame bin limit (rast_types.h
 AUTO_BIG_BIN_TRIS = 8192  # from this many triangles the library picks 32-pixel bins (rast_internal.h)
 
 
-def launches_per_frame(width, height, ntris, tile=0):
-    """8 where a plain frame uses 32-pixel bins, else 7: the library's automatic choice is 32-pixel
-    bins for frames of AUTO_BIG_BIN_TRIS triangles or more, else 16, either one when the other would
-    exceed COUNT_BAND_TILES bins, and 32 for frames where both would. (The numbers are the launches of
-    the pipeline with a tile scan of its own; it takes one fewer now, and 3 for small frames. What
-    a run launches is counted: gpu_launches.)"""
+def bin_edge(width, height, ntris, tile=0):
+    """Bin size of a plain frame in pixels: `tile` where it is one the library takes, else its
+    automatic choice, 32-pixel bins for frames of AUTO_BIG_BIN_TRIS triangles or more, else 16, either
+    one when the other would exceed COUNT_BAND_TILES bins, and 32 for frames where both would."""
     def bins(t):
         return -(-width // t) * -(-height // t)
-    if not (tile in (8, 16, 32) and bins(tile) <= MAX_TILES_PER_FRAME):
-        order = (32, 16) if ntris >= AUTO_BIG_BIN_TRIS else (16, 32)
-        tile = next((t for t in order if bins(t) <= COUNT_BAND_TILES), 32)
-    return 8 if tile == 32 else 7
+    if tile in (8, 16, 32) and bins(tile) <= MAX_TILES_PER_FRAME:
+        return tile
+    order = (32, 16) if ntris >= AUTO_BIG_BIN_TRIS else (16, 32)
+    return next((t for t in order if bins(t) <= COUNT_BAND_TILES), 32)
+
+
+def launches_per_frame(width, height, ntris, tile=0):
+    """8 for 32-pixel bins, else 7: the launches of a frame when the bins had a scan kernel of their own.
+    (One fewer now, and 3 for a small frame; what a run launches is counted: gpu_launches.)"""
+    return 8 if bin_edge(width, height, ntris, tile) == 32 else 7
 
 
 def sustained_point(sweep, bound_ms):
@@ -66,12 +70,12 @@ def sustained_point(sweep, bound_ms):
 
 def batch_tile(scene, tuned):
     """Bin size of a scene in the batch: the autotuned one of its MSAA class, else the library's
-    automatic choice (launches_per_frame)."""
+    automatic choice (bin_edge)."""
     t = tuned.get("msaa%d_tile" % scene.get("msaa", 4), 0)
     if t in (8, 16, 32):
         return t
     from rusterizer_gb300 import scenes
-    return 32 if launches_per_frame(scene["width"], scene["height"], scenes.scene_triangles(scene)) == 8 else 16
+    return bin_edge(scene["width"], scene["height"], scenes.scene_triangles(scene))
 
 
 L2_NOTE = "GPU arm: L2 flushed (256 MB write) before every timed frame"
