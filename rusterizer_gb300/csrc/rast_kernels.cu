@@ -1222,9 +1222,6 @@ __device__ __forceinline__ void store_samples(float* p, const float z[S]) {
     }
 }
 
-template <int S, int TS>
-size_t raster_smem_bytes() { return sizeof(RasterSmem<S, TS>); }
-
 __device__ __forceinline__ uint32_t find_draw(const DrawDev* __restrict__ draws,
                                               const FrameDev& f, uint32_t g) {
     uint32_t lo = f.draw_begin, hi = f.draw_begin + f.draw_count;
@@ -2228,14 +2225,6 @@ cudaError_t launch_raster(const LaunchArgs& a, int msaa, int ts) {
     if (msaa == 4) return rs == 8 ? launch_raster_t<4, 8>(a, nsx) : launch_raster_t<4, 16>(a, nsx);
     if (msaa == 1) return rs == 8 ? launch_raster_t<1, 8>(a, nsx) : launch_raster_t<1, 16>(a, nsx);
     return cudaErrorInvalidValue;
-}
-
-size_t raster_smem(int msaa, int ts) {
-    if (ts != 8 && ts != 16 && ts != 32) return 0;
-    const int rs = raster_edge(ts);
-    if (msaa == 4) return rs == 8 ? raster_smem_bytes<4, 8>() : raster_smem_bytes<4, 16>();
-    if (msaa == 1) return rs == 8 ? raster_smem_bytes<1, 8>() : raster_smem_bytes<1, 16>();
-    return 0;
 }
 
 }  // namespace rast

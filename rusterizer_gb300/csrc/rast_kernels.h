@@ -41,7 +41,6 @@ cudaError_t launch_scans(const LaunchArgs& a);
 cudaError_t launch_bin_scatter(const LaunchArgs& a);
 cudaError_t launch_bin_split(const LaunchArgs& a, int ts);  // 32-pixel bins: before launch_raster
 cudaError_t launch_raster(const LaunchArgs& a, int msaa, int ts);
-size_t raster_smem(int msaa, int ts);
 unsigned long long kernel_launches();
 
 }  // namespace rast

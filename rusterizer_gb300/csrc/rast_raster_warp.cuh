@@ -16,7 +16,6 @@ constexpr int kWarpUnitWarps = 4;  // warps (independent tiles) per CTA of k_ras
 // CTAs per SM the launch bounds aim at: with 4 samples the shared sample tiles allow 5; with
 // one sample registers do (6 would spill)
 constexpr int kWarpUnitCtas = 5;
-constexpr int kWarpUnitCtas1 = 5;
 
 template <int S, int TS>
 struct alignas(16) WarpUnitSmem {
@@ -37,9 +36,6 @@ struct WarpRasterSmem {
     TileQueue tq;
     WarpUnitSmem<S, TS> u[kWarpUnitWarps];
 };
-
-template <int S, int TS>
-size_t warp_raster_smem_bytes() { return sizeof(WarpRasterSmem<S, TS>); }
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v) {
     const uint32_t lane = lane_id();
@@ -502,7 +498,7 @@ __device__ __forceinline__ void warp_unit(WarpUnitSmem<S, TS>& sm, const FrameDe
 // past the heavy classes, times nsx * nsx quadrants, taken one tile per warp from queue[2]; then bins
 // without entries from queue[1], like k_raster.
 template <int S, int TS>
-__global__ void __launch_bounds__(32 * kWarpUnitWarps, S == 1 ? kWarpUnitCtas1 : kWarpUnitCtas) k_raster_warp(const FrameDev* __restrict__ frames,
+__global__ void __launch_bounds__(32 * kWarpUnitWarps, kWarpUnitCtas) k_raster_warp(const FrameDev* __restrict__ frames,
                                                                      int nframes,
                                                                      const uint32_t* __restrict__ order,
                                                                      uint32_t ntotal, uint32_t first_tile,
