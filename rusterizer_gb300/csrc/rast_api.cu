@@ -516,8 +516,8 @@ rast_status rast_mesh_update_async(rast_ctx* c, rast_mesh mesh, const float* pos
         ok = cudaEventRecord(m.used, c->E.stream) == cudaSuccess;
     }
     // the frames already enqueued may still read this mesh: the copies start after the last of them,
-    // beside frames of other meshes (two meshes in turn, 500k triangles at 1080p with readback: 290 -> 281
-    // us a frame; waiting for every frame had put each copy between two frames)
+    // beside frames of other meshes (two meshes in turn, 500k triangles at 1080p with readback: 3% less a
+    // frame; waiting for every frame had put each copy between two frames)
     ok = ok && cudaStreamWaitEvent(c->copy, m.used, 0) == cudaSuccess;
     ok = ok && copy_mesh(m, pos, uv, rgba, idx, c->copy);
     ok = ok && cudaEventRecord(m.ready, c->copy) == cudaSuccess;

@@ -381,8 +381,8 @@ __global__ void __launch_bounds__(256, 6) k_bin_count(const ChunkDev* __restrict
     pdl_enter();
     // per-bin counts of the chunk, two 16-bit counters per word (bin t in half t & 1 of word
     // t / 2): a chunk holds at most 8192 triangles, so no counter carries into its neighbour,
-    // and the histogram of kCountBandTiles = 16384 bins takes 32 KB (6 CTAs per SM by registers: 431 us
-    // a frame against 436 with 8 on the 2M-triangle terrain). Frames with more bins are counted band
+    // and the histogram of kCountBandTiles = 16384 bins takes 32 KB (6 CTAs per SM by registers: with
+    // 8 a frame of the 2M-triangle terrain takes 1% longer). Frames with more bins are counted band
     // by band: the first pass classifies the triangles and stores their boxes, later passes read the boxes back and
     // count the bins of their band (rows of the box outside the band are skipped).
     extern __shared__ uint32_t hist[];
@@ -763,14 +763,15 @@ __global__ void __launch_bounds__(kScatterThreads) k_bin_scatter(
 // Frames of at most kGatherTris triangles (every frame of the run) skip the chunk histograms, the
 // column scan and the scatter: a chunk holds 256 triangles or more, so such a frame has a few chunks
 // and the scatter's CTAs, each serial over its triangles, leave the GPU idle; triangles over many bins
-// make it worse (12 chunks of large triangles at 1440p: 324 us). Here vertices, classification and
+// make it worse (12 chunks of large triangles at 1440p: 324 us in the scatter). Here vertices, classification and
 // clipping are one launch over as many warps as there are triangles to clip, and the bins are
 // filled from the tiles' side: each CTA owns a block of bins and looks at every triangle's box.
-// Measured a frame, before -> now: 3 000 triangles of 32-512 pixels at 1440p 822 -> 478 us, four demo
-// objects at 720p 193 -> 57 us, the cube 97 -> 72 us, soups of 1 000 to 8 000 triangles (1-64 pixels) at
-// 640x480 57 -> 38 .. 93 -> 85 us and at 4K 69 -> 55 .. 168 -> 159 us. Beyond 8 160 triangles the boxes
-// no longer fit shared memory, and the chunks begin to fill the GPU (8 000 small terrain triangles
-// on 640x480 are the one case that the chunk path does better: 54 against 60 us).
+// us a frame among others, by chunks -> so: 3 000 triangles of 32-512 pixels at 1440p 724 -> 437, four demo
+// objects at 720p 159 -> 42, the cube with readback 93 -> 69, soups (1-64 pixels) of 2 000 at 320x240 60 -> 46 and
+// 1080p 84 -> 52, of 8 000 at 1080p 114 -> 92 and 4K 167 -> 161, 64 of them at 640x480 1821 -> 1783. Beyond 8 160
+// triangles the boxes no longer fit shared memory, and the chunks begin to fill the GPU. (Thousands of
+// triangles of a pixel or two on a small image are what the chunks do better: 7 938 of a terrain at 640x480 33
+// against 35 us, at 320x240 43 against 47; of 16-256 pixels there, 505 against 284.)
 
 // The first vertex_blocks CTAs transform 256 vertices each (what the raster reads: screen points); the
 // others take a chunk of 8 `per` triangles, `per` (front_tris: 4, or 10 in a run of many) of them to a
@@ -940,8 +941,10 @@ __device__ __forceinline__ void gather_by_list(const FrameDev& f, uint32_t fi, c
 // counters in the lanes), the bins' ranges are allocated (place_bins), a second pass writes each
 // bin's entries in order. Blocks of 4 x 4 are those of images with few bins, where a block's list may be most of
 // the mesh: from kGatherLong entries on the warps share it (gather_by_list) instead of each walking all of
-// it. 7 938 small triangles, before -> now: at 64x64 149 -> 102 us a frame, at 320x240 64 -> 46, eight such frames at
-// 64x64 235 -> 135; with 512 for kGatherLong 500 triangles at 64x64 take 124 us instead of 121.
+// it. 7 938 triangles of a terrain, walked -> shared: at 64x64 149 -> 102 us a frame, at 320x240 64 -> 46, eight such
+// frames at 64x64 235 -> 135; with 512 for kGatherLong 500 triangles at 64x64 take 124 us instead of 121. Blocks of
+// 8 x 8 stay with the walk: their lists are short, and 64 bins one after another are a longer chain than a quarter
+// row (shared, a 2 000-triangle soup at 1080p takes 60 us instead of 52).
 __global__ void __launch_bounds__(kGatherThreads) k_bin_gather(const FrameDev* __restrict__ frames, int nframes,
                                                                Scratch s) {
     pdl_enter();
@@ -1138,8 +1141,8 @@ __device__ __forceinline__ uint32_t heavy_tiles(const TileQueue& tq, uint32_t he
 
 // Strips of rows that each raster unit is divided into, a CTA (or warp) each, when there are fewer units
 // than places for them: every strip stages all of the unit's entries, so this pays only where the GPU
-// would wait for a few units' serial batches.
-// Returns log2 of their number. A 256-triangle sphere at 256x192: 57 -> 50 us a frame.
+// would wait for a few units' serial batches. Returns log2 of their number. A 256-triangle sphere at
+// 256x192 58 -> 49 us a frame, the cube at 800x600 with readback 74 -> 69.
 __device__ __forceinline__ uint32_t strips_for(uint32_t nunits, uint32_t places) {
     return 4 * nunits <= places ? 2u : 2 * nunits <= places ? 1u : 0u;
 }
@@ -1162,8 +1165,8 @@ struct RasterCfg {
 // neighbours, and a stride of five words keeps eight of them on different bank groups. k_raster is
 // bound by instruction issue and next by shared-memory wavefronts. These records (22 loads before),
 // the span list, the 16-byte depth rounds and the table-free texture filter (tex_argb) together
-// took the 100k-triangle soup at 1080p from 330 to 291 us a frame, 3k large triangles at 1440p
-// from 892 to 835 us and a batch of 20 scenes from 1317 to 1200 us.
+// took 12% off a frame of the 100k-triangle soup at 1080p, 6% off 3k large triangles at 1440p
+// and 9% off a batch of 20 scenes.
 struct RasterItem {
     float4 a;  // p0.x, p0.y, p1.x, p1.y (screen points)
     float4 b;  // p2.x, p2.y, cover_inv, z0
@@ -1478,8 +1481,8 @@ __device__ __forceinline__ void warp_depth(RasterSmem<S, TS>& sm, uint32_t w, ui
     }
     const uint32_t pix = (fr >> 8) & 0xFFu;
     // fragments of one item never share a pixel: most windows over large triangles need no match, whose
-    // time grows with the distinct values (3 000 large triangles at 1440p 473 -> 460 us a frame; no
-    // change on the soups, 0.3% on the 2M-triangle terrain, whose windows mix items)
+    // time grows with the distinct values (3 000 large triangles at 1440p 448 -> 433 us a frame; no
+    // change on the 100k soup, 370 -> 371 on the 2M-triangle terrain, whose windows mix items)
     uint32_t rank = 0, maxr = 0;
     const uint32_t fr0 = __shfl_sync(0xFFFFFFFFu, fr, 0);  // every lane
     if (!__all_sync(0xFFFFFFFFu, (!valid) | (((fr ^ fr0) & 0xFFu) == 0))) {
@@ -1668,8 +1671,8 @@ __global__ void __launch_bounds__(kRasterThreads, kRasterCtasPerSm) k_raster(con
     // unit tickets (heaviest bins first); the next one is taken when the current unit starts its
     // resolve, so the queue update is in flight during the resolve. With no more units than CTAs, CTA
     // i takes unit i and no other: from the counter, the CTAs of the SMs nearest to it take up to
-    // seven before the far ones get any (2 000-triangle soup 86 -> 80 us a frame). With more units the
-    // counter is the better one (a CTA that starts late would hold a heavy unit: 100k soup 290 -> 319).
+    // seven before the far ones get any (2 000-triangle soup with readback 86 -> 81 us a frame). With more
+    // units the counter is the better one (a CTA that starts late would hold a heavy unit: 100k soup 10% slower).
     const uint32_t nwhole = heavy_tiles(sm.tq, frames[0].heavy_bits) * nsub;
     const uint32_t nunits = nwhole << strips_for(nwhole, gridDim.x);
     if (threadIdx.x == 0) sm.misc[6] = strips_for(nwhole, gridDim.x);

@@ -141,7 +141,7 @@ __device__ __forceinline__ void wdepth(WarpUnitSmem<S, TS>& sm, const WItem& my,
         lmeta = shfl_u(my.meta, fr & 31u);
     }
     const uint32_t pix = (fr >> 8) & 0xFFu;
-    // windows of one item need no match (see warp_depth): a captured batch of 20 scenes 1160 -> 1105 us,
+    // windows of one item need no match (see warp_depth): a captured batch of 20 scenes 1087 -> 1040 us,
     // with the same test in the shader
     uint32_t rank = 0, maxr = 0;
     const uint32_t fr0 = __shfl_sync(0xFFFFFFFFu, fr, 0);  // every lane
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(32 * kWarpUnitWarps, kWarpUnitCtas) k_raster_w
     const uint32_t nheavy = heavy_tiles(sh.tq, frames[0].heavy_bits);
     const uint32_t nsub = nsx * nsx;
     // units of the light bins, in strips where they are few. (Strips of the deepest bins, whose length sets
-    // a launch's when it runs alone - 627 -> 519 us for the one-sample scenes of a batch of 20 - cost
+    // a launch's when it runs alone - 17% less for the one-sample scenes of a batch of 20 - cost
     // 1% where the batch's other launch fills the tail, which a mixed batch always has.)
     const uint32_t nwhole = (sh.tq.busy - nheavy) * nsub;
     const uint32_t places = gridDim.x * kWarpUnitWarps;

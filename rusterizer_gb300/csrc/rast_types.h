@@ -97,8 +97,8 @@ constexpr uint32_t kGatherTris = 8160;
 // Triangles per warp of k_front for a run of `tris` triangles: four keep a warp's chain of clipped triangles
 // short while one round of warps takes the run; a larger run fills the GPU either way, and four
 // triangles then leave 20 of a warp's lanes without a corner to transform: 64 frames of 7 938 triangles at
-// 320x240 214 -> 185 us a run with ten (k_front 69 -> 34; 189 with eight), with 65 536 for kFrontFew eight frames of 8 000 take 258 us
-// instead of 248.
+// 320x240 214 -> 185 us a run with ten (k_front 69 -> 34 us; with eight 189). With 65 536 for kFrontFew eight
+// frames of 8 000 at 640x480 take 258 us instead of 248.
 constexpr uint64_t kFrontFew = 16384;
 constexpr uint32_t front_tris(uint64_t tris) { return tris <= kFrontFew ? 4u : 10u; }
 inline uint32_t gather_groups(uint32_t tiles_x, uint32_t tiles_y, uint32_t edge) {
